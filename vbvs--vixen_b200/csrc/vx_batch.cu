@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "vx_cast.cuh"
+#include "vx_regular.cuh"
 
 namespace vx {
 namespace {
@@ -184,7 +185,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_refill_kernel(BatchArgs a) 
     }
 }
 
-template <int BLOCK, int MINB, bool SMEM_STACK>
+// Static lanes.  COUNT: work counters wanted (the general iteration, which
+// keeps them); else cast_plain.
+template <int BLOCK, int MINB, bool SMEM_STACK, bool COUNT>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(BatchArgs a) {
     extern __shared__ uint32_t smem[];
     DevScene* sc = reinterpret_cast<DevScene*>(smem);
@@ -232,13 +235,20 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(BatchArgs a) {
             const float2 p = __ldg(r2), q = __ldg(r2 + 1), w = __ldg(r2 + 2);
             Hit h;
             // no budget: MAX_ITER + 1, which no cast reaches (the loop stops at MAX_ITER)
-            if (!cast_ray_budget<false, !SMEM_STACK, true>(sc[lo], p.x, p.y, q.x, q.y, w.x, w.y, a.tmin, a.tmax, stkN, stkT,
-                                                     cyc, stride, a.budget > 0 ? a.budget : MAX_ITER + 1, h)) {
+            const int budget = a.budget > 0 ? a.budget : MAX_ITER + 1;
+            bool ended;
+            if constexpr (COUNT)
+                ended = cast_ray_budget<false, !SMEM_STACK, true>(sc[lo], p.x, p.y, q.x, q.y, w.x, w.y, a.tmin, a.tmax,
+                                                                  stkN, stkT, cyc, stride, budget, h);
+            else
+                ended = cast_plain(sc[lo], p.x, p.y, q.x, q.y, w.x, w.y, a.tmin, a.tmax, stkN, stkT, cyc, stride,
+                                   budget, h);
+            if (!ended) {
                 a.retry[atomicAdd(a.retry_n, 1u)] = r;
                 continue;
             }
             store_hit(a.hits, out_slot(a, r), h);
-            store_counters(a.counters, out_slot(a, r), h);
+            if constexpr (COUNT) store_counters(a.counters, out_slot(a, r), h);
         }
     }
 }
@@ -654,7 +664,7 @@ struct Variant {
 
 struct vx_batch {
     int device = 0;
-    int per_sm[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // resident blocks per SM of each kernel variant (0 = unresolved)
+    int per_sm[12] = {};  // resident blocks per SM of each kernel variant (0 = unresolved)
     uint32_t S = 0;
     int maxL = 1;
     vx::DevScene* scenes = nullptr;  // device copy of the scene table
@@ -710,18 +720,18 @@ size_t batch_smem(const vx_batch* b, bool smem_stack, int block) {
     return bytes;
 }
 
-template <int BLOCK, int MINB, bool SMEM, bool REFILL>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
 constexpr void (*batch_kernel_ptr())(vx::BatchArgs) {
     if constexpr (REFILL) return vx::batch_refill_kernel<BLOCK, MINB, SMEM>;
-    else return vx::batch_kernel<BLOCK, MINB, SMEM>;
+    else return vx::batch_kernel<BLOCK, MINB, SMEM, COUNT>;
 }
 
 // Resolves (once per batch and variant, outside any stream capture) the
 // dynamic shared-memory attribute and the resident blocks per SM.
-template <int BLOCK, int MINB, bool SMEM, bool REFILL>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
 int prepare_variant(vx_batch* b, int slot) {
     if (b->per_sm[slot]) return VX_OK;
-    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL>();
+    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, COUNT>();
     const size_t smem = batch_smem(b, SMEM, BLOCK);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -735,10 +745,10 @@ int prepare_variant(vx_batch* b, int slot) {
     return VX_OK;
 }
 
-template <int BLOCK, int MINB, bool SMEM, bool REFILL>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
 int launch_variant(vx_batch* b, int slot, const vx::BatchArgs& a, cudaStream_t st) {
-    if (int r = prepare_variant<BLOCK, MINB, SMEM, REFILL>(b, slot)) return r;
-    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL>();
+    if (int r = prepare_variant<BLOCK, MINB, SMEM, REFILL, COUNT>(b, slot)) return r;
+    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, COUNT>();
     kern<<<b->num_sms * b->per_sm[slot], BLOCK, batch_smem(b, SMEM, BLOCK), st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch: launch");
@@ -747,20 +757,27 @@ int launch_variant(vx_batch* b, int slot, const vx::BatchArgs& a, cudaStream_t s
 
 template <bool PREPARE_ONLY>
 int dispatch_batch(vx_batch* b, const vx_batch_tuning& t, const vx::BatchArgs* a, cudaStream_t st) {
-    const int slot = (t.block == 128 ? 0 : 4) + (t.stack_in_shared ? 0 : 2) + (t.refill ? 1 : 0);
-#define VX_BATCH_CASE(SLOT, BLK, MINB, SMEM, REF)                                                      \
+    // the refilling kernels keep counters in any case; static lanes have a counting form of their own
+    const int slot = (!t.refill && a && a->counters)
+                         ? 8 + (t.block == 128 ? 0 : 2) + (t.stack_in_shared ? 0 : 1)
+                         : (t.block == 128 ? 0 : 4) + (t.stack_in_shared ? 0 : 2) + (t.refill ? 1 : 0);
+#define VX_BATCH_CASE(SLOT, BLK, MINB, SMEM, REF, CNT)                                                 \
     case SLOT:                                                                                          \
-        return PREPARE_ONLY ? prepare_variant<BLK, MINB, SMEM, REF>(b, SLOT)                            \
-                            : launch_variant<BLK, MINB, SMEM, REF>(b, SLOT, *a, st);
+        return PREPARE_ONLY ? prepare_variant<BLK, MINB, SMEM, REF, CNT>(b, SLOT)                       \
+                            : launch_variant<BLK, MINB, SMEM, REF, CNT>(b, SLOT, *a, st);
     switch (slot) {
-        VX_BATCH_CASE(0, 128, 6, true, false)
-        VX_BATCH_CASE(1, 128, 4, true, true)
-        VX_BATCH_CASE(2, 128, 6, false, false)
-        VX_BATCH_CASE(3, 128, 4, false, true)
-        VX_BATCH_CASE(4, 256, 3, true, false)
-        VX_BATCH_CASE(5, 256, 2, true, true)
-        VX_BATCH_CASE(6, 256, 3, false, false)
-        VX_BATCH_CASE(7, 256, 2, false, true)
+        VX_BATCH_CASE(0, 128, 6, true, false, false)
+        VX_BATCH_CASE(1, 128, 4, true, true, true)
+        VX_BATCH_CASE(2, 128, 6, false, false, false)
+        VX_BATCH_CASE(3, 128, 4, false, true, true)
+        VX_BATCH_CASE(4, 256, 3, true, false, false)
+        VX_BATCH_CASE(5, 256, 2, true, true, true)
+        VX_BATCH_CASE(6, 256, 3, false, false, false)
+        VX_BATCH_CASE(7, 256, 2, false, true, true)
+        VX_BATCH_CASE(8, 128, 6, true, false, true)
+        VX_BATCH_CASE(9, 128, 6, false, false, true)
+        VX_BATCH_CASE(10, 256, 3, true, false, true)
+        VX_BATCH_CASE(11, 256, 3, false, false, true)
     }
 #undef VX_BATCH_CASE
     return fail(VX_EINVAL, "vx_cast_batch: no kernel variant for this tuning");
@@ -1499,7 +1516,7 @@ int noalloc_setup(int dev, NoallocDevice*& out) {
         void* ptr = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: cudaGetSymbolAddress");
-        auto kern = batch_kernel<256, 3, true>;
+        auto kern = batch_kernel<256, 3, true, false>;
         const size_t smem_max = size_t(VX_NOALLOC_MAX_SCENES) * sizeof(DevScene) +
                                 ((size_t(VX_NOALLOC_MAX_SCENES) + 1 + 3) & ~size_t(3)) * 4 +
                                 (size_t(2) * MAX_LEVELS_ALL + CYC_WORDS) * 256 * 4;
@@ -1560,7 +1577,7 @@ static int vx_cast_batch_noalloc_body(const vx_scene* const* scenes, uint32_t co
                 tmax, hits, nullptr, reinterpret_cast<uint32_t*>(d->scratch), 32u, maxL};
     const size_t smem = size_t(count) * sizeof(DevScene) + ((size_t(count) + 1 + 3) & ~size_t(3)) * 4 +
                         (size_t(2) * size_t(maxL) + CYC_WORDS) * 256 * 4;
-    batch_kernel<256, 3, true><<<d->blocks, 256, smem, st>>>(a);
+    batch_kernel<256, 3, true, false><<<d->blocks, 256, smem, st>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: launch");
     return VX_OK;

@@ -22,6 +22,7 @@
 // target costs one atomicAdd per channel per warp.
 
 #include "vx_cast.cuh"
+#include "vx_regular.cuh"
 
 namespace vx {
 namespace {
@@ -63,7 +64,7 @@ __device__ __forceinline__ void forward_pixel(const DevScene& s, const CameraDev
     float uv_y;
     camera_ray(cam, px, py, w, hgt, r, &uv_y);
     Hit h;
-    cast_ray(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, stride, h);
+    cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, stride, MAX_ITER + 1, h);
     store_hit(record, i, h);
     float c[3];
     if (h.flags & F_HIT) {
@@ -102,7 +103,7 @@ constexpr int FWD_WARPS = VX_DIFF_FWD_WARPS;
 constexpr int FWD_THREADS = VX_DIFF_TILED ? FWD_WARPS * 32 : DBLOCK;
 
 __global__ void __launch_bounds__(FWD_THREADS, 768 / FWD_THREADS) diff_forward_kernel(
-    DevScene s, Views views, uint32_t nviews, uint32_t w, uint32_t hgt, int kind, const float* __restrict__ attr,
+    const __grid_constant__ DevScene s, Views views, uint32_t nviews, uint32_t w, uint32_t hgt, int kind, const float* __restrict__ attr,
     const uint32_t* __restrict__ idx, float* __restrict__ image, vx_hit* __restrict__ record) {
     extern __shared__ uint32_t smem[];
     uint32_t* stkN = smem + threadIdx.x;

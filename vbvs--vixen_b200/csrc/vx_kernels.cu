@@ -1,5 +1,6 @@
 // vx_kernels.cu - plain (one launch per scene) cast and render kernels.
 #include "vx_cast.cuh"
+#include "vx_regular.cuh"
 #include "vx_palette.h"
 
 namespace vx {
@@ -22,8 +23,8 @@ constexpr int RENDER_THREADS = RENDER_WARPS * 32;
 // 0.1249 ms).
 constexpr int CAST_MIN_BLOCKS = 896 / BLOCK;
 
-template <bool LOD>
-__global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(DevScene s, const vx_ray* __restrict__ rays, uint32_t n,
+template <bool LOD, bool COUNT>
+__global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays, uint32_t n,
                                                       float tmin, float tmax, vx_hit* __restrict__ hits,
                                                       void* __restrict__ color,
                                                       vx_ray_counters* __restrict__ counters, LodCone lod) {
@@ -36,10 +37,11 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(DevScene s
     const float2* r2 = reinterpret_cast<const float2*>(rays + i);
     const float2 a = __ldg(r2), b = __ldg(r2 + 1), c = __ldg(r2 + 2);
     Hit h;
-    cast_ray<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h, lod);
+    if constexpr (COUNT) cast_ray<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h, lod);
+    else cast_plain<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, MAX_ITER + 1, h, lod);
     store_hit(hits, i, h);
     if (color) store_color(s, color, i, h);
-    if (counters) {
+    if constexpr (COUNT) {
         uint4 rc;
         rc.x = (h.iters & 0xFFFFu) | (h.grid_reads << 16);
         rc.y = h.dda_steps;
@@ -52,7 +54,7 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(DevScene s
 // The cast of rays compacted on the device: `count` (device) rays of at most
 // n_max, the hit record of ray i going to slot map[i].  The per-ray work is
 // cast_kernel's (castRay, no colour or counters).
-__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(DevScene s, const vx_ray* __restrict__ rays,
+__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays,
                                                                         uint32_t n_max, const uint32_t* __restrict__ count,
                                                                         const uint32_t* __restrict__ map, float tmin,
                                                                         float tmax, vx_hit* __restrict__ hits) {
@@ -65,7 +67,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(DevScen
     const float2* r2 = reinterpret_cast<const float2*>(rays + i);
     const float2 a = __ldg(r2), b = __ldg(r2 + 1), c = __ldg(r2 + 2);
     Hit h;
-    cast_ray(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h);
+    cast_plain(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, MAX_ITER + 1, h);
     store_hit(hits, __ldg(map + i), h);
 }
 
@@ -75,7 +77,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(DevScen
 // along a row.  Warp task t is piece t & 7 of tile t >> 3; a block holds
 // RENDER_WARPS consecutive tasks.  Outputs are indexed by pixel (y * w + x).
 __global__ void __launch_bounds__(RENDER_THREADS, 768 / RENDER_THREADS) render_kernel(
-    DevScene s, CameraDev cam, uint32_t w, uint32_t hgt, uint32_t* __restrict__ image, vx_hit* __restrict__ hits,
+    const __grid_constant__ DevScene s, CameraDev cam, uint32_t w, uint32_t hgt, uint32_t* __restrict__ image, vx_hit* __restrict__ hits,
     void* __restrict__ color) {
     extern __shared__ uint32_t smem[];
     uint32_t* stkN = smem + threadIdx.x;
@@ -93,7 +95,7 @@ __global__ void __launch_bounds__(RENDER_THREADS, 768 / RENDER_THREADS) render_k
     float uv_y;
     camera_ray(cam, px, py, w, hgt, r, &uv_y);
     Hit h;
-    cast_ray(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, RENDER_THREADS, h);
+    cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, RENDER_THREADS, MAX_ITER + 1, h);
     if (hits) store_hit(hits, i, h);
     if (color) store_color(s, color, i, h);
     if (image) {
@@ -170,15 +172,12 @@ int launch_cast(const DevScene& s, const vx_ray* rays, uint32_t n, float tmin, f
     const uint32_t grid = (n + BLOCK - 1) / BLOCK;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t smem = stack_bytes(s, BLOCK);
-    if (lod && lod->ray_dir_size > 0.0f) {
-        if (cudaError_t e = allow_smem(cast_kernel<true>, smem)) return int(e);
-        cast_kernel<true><<<grid, BLOCK, smem, st>>>(s, rays, n, tmin, tmax, hits, color, counters,
-                                                     LodCone{lod->ray_orig_size, lod->ray_dir_size});
-    } else {
-        if (cudaError_t e = allow_smem(cast_kernel<false>, smem)) return int(e);
-        cast_kernel<false><<<grid, BLOCK, smem, st>>>(s, rays, n, tmin, tmax, hits, color, counters,
-                                                      LodCone{0.0f, 0.0f});
-    }
+    const bool cone = lod && lod->ray_dir_size > 0.0f;
+    const LodCone lc = cone ? LodCone{lod->ray_orig_size, lod->ray_dir_size} : LodCone{0.0f, 0.0f};
+    auto* kernel = cone ? (counters ? cast_kernel<true, true> : cast_kernel<true, false>)
+                        : (counters ? cast_kernel<false, true> : cast_kernel<false, false>);
+    if (cudaError_t e = allow_smem(kernel, smem)) return int(e);
+    kernel<<<grid, BLOCK, smem, st>>>(s, rays, n, tmin, tmax, hits, color, counters, lc);
     return int(cudaGetLastError());
 }
 
