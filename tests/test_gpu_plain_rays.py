@@ -98,3 +98,18 @@ def test_plain_rays_batched_equal_oracle(vx, vo, cuda, tuning):
     assert_hits_equal(g[:20011], oracles[0].cast_rays(parts[0]), None, "scene 0")
     assert_hits_equal(g[20011:], oracles[1].cast_rays(parts[1]), None, "scene 1")
     batch.close()
+
+
+def test_bricks_away_from_their_slots(vx, vo, cuda):
+    """A scene whose grid slots name bricks with other coordinates is accepted; its casts march the
+    brick's own box, with and without counters."""
+    wmin, wmax, depth, count = SCENES[0]
+    o = sparse_scene(vo, wmin, wmax, depth, 12, count)
+    a = scene_from_oracle(vx, o, (wmin, wmax), depth)
+    a.brick_coord = np.roll(a.brick_coord, 3)
+    scene = vx.Scene(a)
+    rays = edge_rays(wmin, wmax, 20001, 13)
+    plain, _, _ = gpu_cast(vx, scene, rays, with_counters=False)
+    general, _, _ = gpu_cast(vx, scene, rays, with_counters=True)
+    np.testing.assert_array_equal(plain, general)
+    assert (plain["flags"] & 1).any()

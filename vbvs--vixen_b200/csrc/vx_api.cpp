@@ -242,6 +242,19 @@ int vx_scene_create(const vx_scene_desc* d, vx_scene** out) {
             return vx::cuda_fail(e, "vx_scene_create: cudaMemcpy");
         }
     }
+    if (s->dev.ordinary) {
+        // the pool's last 256 bytes are spare: the check's result goes there
+        uint32_t* mismatch = reinterpret_cast<uint32_t*>(static_cast<char*>(s->pool) + s->pool_bytes - 256);
+        uint32_t bad = 0;
+        cudaError_t e = cudaMemset(mismatch, 0, 4);
+        if (e == cudaSuccess) e = cudaError_t(vx::launch_grid_check(s->dev, mismatch, nullptr));
+        if (e == cudaSuccess) e = cudaMemcpy(&bad, mismatch, 4, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) {
+            vx_scene_destroy(s);
+            return vx::cuda_fail(e, "vx_scene_create: grid check");
+        }
+        if (bad) s->dev.ordinary = 0;
+    }
     *out = s;
     return VX_OK;
 }

@@ -102,7 +102,7 @@ __device__ __forceinline__ void forward_pixel(const DevScene& s, const CameraDev
 constexpr int FWD_WARPS = VX_DIFF_FWD_WARPS;
 constexpr int FWD_THREADS = VX_DIFF_TILED ? FWD_WARPS * 32 : DBLOCK;
 
-__global__ void __launch_bounds__(FWD_THREADS, 768 / FWD_THREADS) diff_forward_kernel(
+__global__ void __launch_bounds__(FWD_THREADS, 1024 / FWD_THREADS) diff_forward_kernel(
     const __grid_constant__ DevScene s, Views views, uint32_t nviews, uint32_t w, uint32_t hgt, int kind, const float* __restrict__ attr,
     const uint32_t* __restrict__ idx, float* __restrict__ image, vx_hit* __restrict__ record) {
     extern __shared__ uint32_t smem[];

@@ -1,4 +1,6 @@
 // vx_kernels.cu - plain (one launch per scene) cast and render kernels.
+#include <algorithm>
+
 #include "vx_cast.cuh"
 #include "vx_regular.cuh"
 #include "vx_palette.h"
@@ -17,11 +19,12 @@ namespace {
 constexpr int BLOCK = VX_CAST_BLOCK;
 constexpr int RENDER_WARPS = VX_RENDER_WARPS;
 constexpr int RENDER_THREADS = RENDER_WARPS * 32;
-// Resident blocks per SM the cast kernel is compiled for: 14 blocks of 64
-// threads leave 72 registers a thread (cfg2 frame 0.1208 -> 0.1188 ms against
-// 12 blocks at 80 registers; 16 blocks at 64 registers spill and measure
-// 0.1249 ms).
-constexpr int CAST_MIN_BLOCKS = 896 / BLOCK;
+// Threads per SM the cast and render kernels are compiled for: 1,024 leave 64
+// registers a thread.  At 768 / 896 / 1,024 / 1,280 threads the 1080p cave frame
+// takes 145 / 143 / 139 / 155 us, the 4K city frame with shadow rays 1.13 / 1.08 /
+// 1.05 / 1.17 ms (more warps to issue from, until spills cost more).
+constexpr int CAST_THREADS = 1024;
+constexpr int CAST_MIN_BLOCKS = CAST_THREADS / BLOCK;
 
 template <bool LOD, bool COUNT>
 __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays, uint32_t n,
@@ -54,7 +57,7 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __gr
 // The cast of rays compacted on the device: `count` (device) rays of at most
 // n_max, the hit record of ray i going to slot map[i].  The per-ray work is
 // cast_kernel's (castRay, no colour or counters).
-__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays,
+__global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_mapped_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays,
                                                                         uint32_t n_max, const uint32_t* __restrict__ count,
                                                                         const uint32_t* __restrict__ map, float tmin,
                                                                         float tmax, vx_hit* __restrict__ hits) {
@@ -76,7 +79,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) cast_mapped_kernel(const _
 // neighbours in both image directions, so their traversals diverge less than
 // along a row.  Warp task t is piece t & 7 of tile t >> 3; a block holds
 // RENDER_WARPS consecutive tasks.  Outputs are indexed by pixel (y * w + x).
-__global__ void __launch_bounds__(RENDER_THREADS, 768 / RENDER_THREADS) render_kernel(
+__global__ void __launch_bounds__(RENDER_THREADS, CAST_THREADS / RENDER_THREADS) render_kernel(
     const __grid_constant__ DevScene s, CameraDev cam, uint32_t w, uint32_t hgt, uint32_t* __restrict__ image, vx_hit* __restrict__ hits,
     void* __restrict__ color) {
     extern __shared__ uint32_t smem[];
@@ -144,6 +147,14 @@ __global__ void __launch_bounds__(RENDER_THREADS, 768 / RENDER_THREADS) render_k
     }
 }
 
+__global__ void __launch_bounds__(256) grid_check_kernel(DevScene s, uint32_t* __restrict__ mismatch) {
+    const uint32_t bpa = uint32_t(s.bpa), slots = bpa * bpa * bpa;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
+        const uint32_t b = __ldg(s.grid + i);
+        if (b != NONE && __ldg(s.coord + b) != (i % bpa | (i / bpa % bpa) << 10 | (i / (bpa * bpa)) << 20)) *mismatch = 1u;
+    }
+}
+
 __global__ void camera_rays_kernel(CameraDev cam, uint32_t w, uint32_t hgt, vx_ray* __restrict__ rays) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= w * hgt) return;
@@ -202,6 +213,13 @@ int launch_render(const DevScene& s, const CameraDev& cam, uint32_t w, uint32_t 
     if (cudaError_t e = allow_smem(render_kernel, smem)) return int(e);
     render_kernel<<<uint32_t(grid), RENDER_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(s, cam, w, h, image, hits,
                                                                                         color);
+    return int(cudaGetLastError());
+}
+
+int launch_grid_check(const DevScene& s, uint32_t* mismatch, void* stream) {
+    const uint64_t slots = uint64_t(s.bpa) * uint64_t(s.bpa) * uint64_t(s.bpa);
+    grid_check_kernel<<<uint32_t(std::min<uint64_t>((slots + 255) / 256, 148 * 8)), 256, 0,
+                        static_cast<cudaStream_t>(stream)>>>(s, mismatch);
     return int(cudaGetLastError());
 }
 

@@ -39,11 +39,15 @@
 //    a ray that is not regular can take, leaves everything but t_min as it was:
 //    when t_min stays too, the state repeats.)
 //
-// Bound: instruction issue.  Measured against the general iteration (B200):
-// 1024^3 cave, 1920 x 1080 primary rays 239 -> 143 us; 2048^3 city at 4K with
-// shadow rays 1.65 -> 1.09 ms; 1,000,003 incoherent rays with LOD 308 -> 228 us;
-// 24-scene batched frame, primary pass 1.24 -> 0.80 ms (942 M -> 602 M warp
-// instructions), bounce pass 1.77 -> 1.38 ms.
+// Bound: instruction issue, and in launches of few warps the dependent steps of
+// the longest one (descriptor, slot, voxels; then one voxel after the other).
+// Measured against the general iteration (B200): 1024^3 cave, 1920 x 1080 primary
+// rays 239 -> 120 us; 512 x 512 rays in pixel rows through a 256^3 scene
+// 123 -> 55 us; 2048^3 city at 4K with shadow rays 1.65 -> 1.05 ms; 1,000,003
+// incoherent rays with LOD 308 -> 222 us; 24-scene batched frame, primary pass
+// 1.24 -> 0.71 ms (942 M -> 570 M warp instructions), bounce pass 1.77 -> 1.22 ms.
+// Of this the branch-free march over bricks whose coordinates come from their
+// slot took 86 -> 55 us, 139 -> 120 us and 2.72 -> 2.46 ms per frame.
 #pragma once
 #include "vx_cast.cuh"
 
@@ -124,10 +128,9 @@ __device__ __forceinline__ void regular_hit(const RegRay& r, const float vmn[3],
 // of the brick sets bit 3 of its field); one 8-byte load gives the 64 voxels
 // of a slice, read again when z steps.
 template <bool REG>
-__device__ __forceinline__ bool regular_brick(const DevScene& s, uint32_t brick, const RegRay& r, Hit& h) {
-    const uint32_t bc = __ldg(s.coord + bounded(brick, s.brick_count, V_BRICK));
-    const float bmn[3] = {small_float((bc << 3) & 0x1FF8u), small_float((bc >> 7) & 0x1FF8u),
-                          small_float((bc >> 17) & 0x1FF8u)};
+__device__ __forceinline__ bool regular_brick(const DevScene& s, uint32_t brick, const uint32_t slot[3],
+                                              const RegRay& r, Hit& h) {
+    const float bmn[3] = {small_float(slot[0] * 8u), small_float(slot[1] * 8u), small_float(slot[2] * 8u)};
     float tn[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) tn[i] = ((r.rcp[i] > 0.0f ? bmn[i] : bmn[i] + 8.0f) - r.lo[i]) * r.rcp[i];
@@ -165,40 +168,38 @@ __device__ __forceinline__ bool regular_brick(const DevScene& s, uint32_t brick,
         for (int i = 0; i < 3; ++i) tNext[i] = still<REG>(r.d[i]) ? FLT_MAX_ : tMin + a[i] / r.d[i];
     }
     uint32_t p = c[0] | (c[1] << 4) | (c[2] << 8);
+    const uint32_t sx = r.d[0] > 0.0f ? 1u : ~0u, sy = r.d[1] > 0.0f ? 16u : ~15u, sz = r.d[2] > 0.0f ? 256u : ~255u;
+    // Branch-free over the axes: the smallest tNext is the one the reference's
+    // comparisons pick (ties go to z, then y), and lanes that step along
+    // different axes stay together.
     for (;;) {
-        if (tNext[0] < tNext[1] && tNext[0] < tNext[2]) {
-            if (tNext[0] > tMax) return false;
-            p += r.d[0] > 0.0f ? 1u : ~0u;
-            tNext[0] += fabsf(r.rcp[0]);
-            if (p & 0x8u) return false;
-        } else if (tNext[1] < tNext[2]) {
-            if (tNext[1] > tMax) return false;
-            p += r.d[1] > 0.0f ? 16u : ~15u;
-            tNext[1] += fabsf(r.rcp[1]);
-            if (p & 0x80u) return false;
-        } else {
-            if (tNext[2] > tMax) return false;
-            p += r.d[2] > 0.0f ? 256u : ~255u;
-            tNext[2] += fabsf(r.rcp[2]);
-            if (p & 0x800u) return false;
-            w = __ldg(occ + (p >> 8));
-        }
-        if (((p & 0x40u ? w.y : w.x) >> ((p & 7u) | ((p >> 1) & 0x18u))) & 1u) {
-            vmn[0] = bmn[0] + small_float(p & 7u);
-            vmn[1] = bmn[1] + small_float((p >> 4) & 7u);
-            vmn[2] = bmn[2] + small_float(p >> 8);
-            regular_hit<REG>(r, vmn, (p & 7u) | ((p >> 1) & 0x38u) | ((p >> 2) & 0x1C0u), h);
-            return true;
-        }
+        if (nmin3(tNext[0], tNext[1], tNext[2]) > tMax) return false;
+        const bool ax = tNext[0] < tNext[1] && tNext[0] < tNext[2];
+        const bool ay = !ax && tNext[1] < tNext[2];
+        const bool az = !ax && !ay;
+        p += ax ? sx : (ay ? sy : sz);
+        if (ax) tNext[0] += fabsf(r.rcp[0]);
+        if (ay) tNext[1] += fabsf(r.rcp[1]);
+        if (az) tNext[2] += fabsf(r.rcp[2]);
+        if (p & 0x888u) return false;
+        if (az) w = __ldg(occ + (p >> 8));
+        if (((p & 0x40u ? w.y : w.x) >> ((p & 7u) | ((p >> 1) & 0x18u))) & 1u) break;
     }
+    vmn[0] = bmn[0] + small_float(p & 7u);
+    vmn[1] = bmn[1] + small_float((p >> 4) & 7u);
+    vmn[2] = bmn[2] + small_float(p >> 8);
+    regular_hit<REG>(r, vmn, (p & 7u) | ((p >> 1) & 0x38u) | ((p >> 2) & 0x1C0u), h);
+    return true;
 }
 
-// Index of the brick slot at box position i in [0.001, 0.999]^3 (the lookups
-// of handleLeafHit): min(i * wsize, wsize - 0.001) / 8 truncated, at most bpa - 1.
-__device__ __forceinline__ uint32_t regular_lookup(const DevScene& s, float x, float y, float z) {
+// The brick slot at grid position x (a lookup of handleLeafHit): x / 8
+// truncated, at most bpa - 1.  Returns its brick; DevScene::ordinary says that
+// a slot's brick has the slot's coordinates, so they need not be loaded.
+__device__ __forceinline__ uint32_t regular_lookup(const DevScene& s, const float x[3], uint32_t slot[3]) {
     const int bmax = s.bpa - 1;
-    return grid_lookup(s, imin(f2i_in_range(x * 0.125f), bmax), imin(f2i_in_range(y * 0.125f), bmax),
-                       imin(f2i_in_range(z * 0.125f), bmax));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) slot[i] = uint32_t(imin(int(trunc_bits(x[i] * 0.125f) & 0x7FFFFFu), bmax));
+    return grid_lookup(s, int(slot[0]), int(slot[1]), int(slot[2]));
 }
 
 // Long cycles: checkpoints of the POP state (w[0..6]), the pushed mask and the
@@ -368,7 +369,8 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
                     }
                     x[i] = nmin(nclamp(b, 0.001f, 0.999f) * s.wsize[i], s.wsm[i]);
                 }
-                uint32_t brick = regular_lookup(s, x[0], x[1], x[2]);
+                uint32_t slot[3];
+                uint32_t brick = regular_lookup(s, x, slot);
                 uint32_t method = 1u << 4;
                 if (brick == NONE) {
                     method = 2u << 4;
@@ -377,7 +379,7 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
 #pragma unroll
                         for (int i = 0; i < 3; ++i)
                             x[i] = nclamp(((o[i] + r.d[i] * te0) - s.wmin[i]) + r.d[i] * 0.01f, 0.0f, s.wsm[i]);
-                        entry_brick = regular_lookup(s, x[0], x[1], x[2]);
+                        entry_brick = regular_lookup(s, x, slot);
                     }
                     brick = entry_brick;
                     if (brick == NONE) {
@@ -388,13 +390,19 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
                             const uint32_t ci = nd.x + __popc(valid & ~leafs) + __popc(leafs & ((1u << idxw) - 1u));
                             if (ci < s.node_count) {
                                 const uint32_t b = __ldg(s.node_brick + ci);
-                                if (b < s.brick_count) brick = b;
+                                if (b < s.brick_count) {
+                                    brick = b;
+                                    const uint32_t bc = __ldg(s.coord + b);
+                                    slot[0] = bc & 0x3FFu;
+                                    slot[1] = (bc >> 10) & 0x3FFu;
+                                    slot[2] = (bc >> 20) & 0x3FFu;
+                                }
                             }
                         }
                     }
                 }
                 if (brick < ENTRY_MISSED) {
-                    if (regular_brick<REG>(s, brick, r, h)) {
+                    if (regular_brick<REG>(s, brick, slot, r, h)) {
                         h.brick = brick;
                         h.node = parent;
                         h.flags |= method;
