@@ -12,3 +12,18 @@ def test_device_noise_equals_host(vx, cuda, R, spacing, octaves, fill, shell):
     host = vx.synth_noise(R, spacing, octaves, fill, 1234, shell)
     dev = vx.synth_noise_dev(R, spacing, octaves, fill, 1234, shell).cpu().numpy().view(np.uint64)
     np.testing.assert_array_equal(dev, host)
+
+
+@pytest.mark.parametrize("R,spacing,octaves,fill,shell", [
+    (192, 12, 3, 0.3, False),       # rows side by side in a block leave threads over
+    (320, 20, 3, 0.37, True),       # the last segment of a row is short
+    (64, 1, 1, 0.5, False),         # one lattice cell per voxel
+    (128, 1 << 15, 16, 0.25, True),  # the most octaves, the coarsest far larger than the grid
+    (128, 256, 9, 0.62, False),
+    (64, 1 << 30, 1, 0.5, False),   # nearly all values alike: more values in one bin than candidates
+    (64, 1 << 20, 2, 0.001, False), (128, 8, 3, 1e-7, False), (64, 5, 2, 0.9999, True)])
+def test_device_noise_edges_equal_host(vx, cuda, R, spacing, octaves, fill, shell):
+    """Odd tile shapes, every register form (4, 8, 16 octaves), both ways to the threshold."""
+    host = vx.synth_noise(R, spacing, octaves, fill, 99, shell)
+    dev = vx.synth_noise_dev(R, spacing, octaves, fill, 99, shell).cpu().numpy().view(np.uint64)
+    np.testing.assert_array_equal(dev, host)
