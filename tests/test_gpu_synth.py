@@ -27,3 +27,12 @@ def test_device_noise_edges_equal_host(vx, cuda, R, spacing, octaves, fill, shel
     host = vx.synth_noise(R, spacing, octaves, fill, 99, shell)
     dev = vx.synth_noise_dev(R, spacing, octaves, fill, 99, shell).cpu().numpy().view(np.uint64)
     np.testing.assert_array_equal(dev, host)
+
+
+@pytest.mark.parametrize("spacing,octaves,fill", [(32, 3, 0.1), (32, 3, 0.37), (27, 2, 0.1)])
+def test_device_noise_rounds_like_the_host(vx, cuda, spacing, octaves, fill):
+    """134 M voxels: several per binary32 value, so a value off by one unit in the last place near
+    the threshold changes bits (products and sums fused into one rounding change tens of them)."""
+    host = vx.synth_noise(512, spacing, octaves, fill, 5, False)
+    dev = vx.synth_noise_dev(512, spacing, octaves, fill, 5, False).cpu().numpy().view(np.uint64)
+    np.testing.assert_array_equal(dev, host)

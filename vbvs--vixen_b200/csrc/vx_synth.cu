@@ -23,6 +23,7 @@
 
 #include "vx_hash.h"
 #include "vx_internal.h"
+#include "vx_pairs.cuh"
 
 namespace vx {
 namespace {
@@ -47,6 +48,7 @@ struct OctDev {
 };
 struct NoiseParams {
     uint32_t R, octaves, row_cells, rows;  // row_cells: cells of all octaves; rows: of a tile (8, or 4 when 8 do not fit)
+    float neg_zero;       // -0 (vx_pairs.cuh)
     const uint2* column;  // [octave][x]: place in a row's cells, weight along x
     OctDev oct[MAX_OCT];
 };
@@ -88,10 +90,6 @@ __global__ void lattice_kernel(NoiseParams p, float* lat, uint64_t total, uint2*
         column[t] = make_uint2(p.oct[o].first + cell, __float_as_uint(w));
     }
 }
-
-// Two values at once (add.f32x2 and the like): each half is rounded as the
-// scalar operation rounds it.  b - a is fma(a, -1, b): the product is exact.
-__device__ __forceinline__ float2 sub2(float2 b, float2 a) { return __ffma2_rn(a, make_float2(-1.0f, -1.0f), b); }
 
 // The values of all voxels, tile by tile (p.rows rows of one z slice, all
 // columns).  use(bits, x, y, z, word) gets the bit patterns of four rows y ..
@@ -177,9 +175,9 @@ __device__ __forceinline__ void for_each_value(const NoiseParams& p, float4* cel
                             const float2 amp = make_float2(p.oct[o].amp, p.oct[o].amp);
 #pragma unroll
                             for (int k = 0; k < 2; ++k) {
-                                const float2 v = __fadd2_rn(a2[k], __fmul2_rn(wx[o], sub2(b2[k], a2[k])));
+                                const float2 v = __fadd2_rn(a2[k], mul2(wx[o], sub2(b2[k], a2[k]), p.neg_zero));
                                 // octave 0 has amplitude 1: 0 + 1 * v is v (no value is -0)
-                                out[k] = o == 0 ? v : __fadd2_rn(out[k], __fmul2_rn(amp, v));
+                                out[k] = o == 0 ? v : __fadd2_rn(out[k], mul2(amp, v, p.neg_zero));
                             }
                         }
                     const uint32_t bits[4] = {__float_as_uint(out[0].x), __float_as_uint(out[0].y),
@@ -384,6 +382,7 @@ static int vx_synth_noise_dev_body(uint32_t R, uint32_t spacing, uint32_t octave
     NoiseParams p{};
     p.R = R;
     p.octaves = octaves;
+    p.neg_zero = -0.0f;
     // one allocation: histograms, the select's state, the lattices (each at a
     // multiple of 64 floats), the candidates
     const uint64_t o_low = HIST_BINS * sizeof(unsigned long long), o_sel = o_low + LOW_BINS * 4;
