@@ -175,20 +175,31 @@ VX_HD uint32_t row8(const uint32_t* occ, int y, int z) {
     return (occ[2 * z + (y >> 2)] >> ((y & 3) * 8)) & 0xFFu;
 }
 
-// Neighbour codes of the 16 texels of block `block` (voxels block*16 ..
-// block*16 + 15: rows y = 2p and 2p + 1 of slice z, p = block & 3,
-// z = block >> 2).  Returns whether any texel is occupied.
-VX_HD bool block_codes(const uint32_t* occ, int block, uint8_t* code) {
+// What a block's encoding depends on, in 64 bits: its two occupancy rows (y =
+// 2p and 2p + 1 of slice z, p = block & 3, z = block >> 2; voxels block*16 ..
+// block*16 + 15) and the neighbour bits that reach an occupied voxel, a byte
+// per row: {row 0, row 1, row y0 - 1, row y0 + 2, rows z + 1, rows z - 1}.
+// z neighbours present on both sides cancel in the central difference and are
+// left out.  0 for a block without occupied texels.
+VX_HD uint64_t block_key(const uint32_t* occ, int block) {
     const int z = block >> 2, y0 = (block & 3) * 2;
-    bool any = false;
+    const uint32_t r0 = row8(occ, y0, z), r1 = row8(occ, y0 + 1, z);
+    const uint32_t rows = r0 | (r1 << 8);
+    const uint32_t zp = (row8(occ, y0, z + 1) | (row8(occ, y0 + 1, z + 1) << 8)) & rows;
+    const uint32_t zm = (row8(occ, y0, z - 1) | (row8(occ, y0 + 1, z - 1) << 8)) & rows;
+    const uint32_t lo = rows | ((row8(occ, y0 - 1, z) & r0) << 16) | ((row8(occ, y0 + 2, z) & r1) << 24);
+    return uint64_t(lo) | (uint64_t((zp & ~zm) | ((zm & ~zp) << 16)) << 32);
+}
+
+// Neighbour codes of the 16 texels of the block with this key.
+VX_HD void key_codes(uint64_t key, uint8_t* code) {
+    const uint32_t lo = uint32_t(key), hi = uint32_t(key >> 32);
     VX_UNROLL
     for (int r = 0; r < 2; ++r) {
-        const int y = y0 + r;
-        const uint32_t row = row8(occ, y, z);
-        any = any || row != 0u;
+        const uint32_t row = (lo >> (8 * r)) & 0xFFu;
         const uint32_t xp = row >> 1, xm = (row << 1) & 0xFFu;
-        const uint32_t yp = row8(occ, y + 1, z), ym = row8(occ, y - 1, z);
-        const uint32_t zp = row8(occ, y, z + 1), zm = row8(occ, y, z - 1);
+        const uint32_t yp = r == 0 ? (lo >> 8) & 0xFFu : lo >> 24, ym = r == 0 ? (lo >> 16) & 0xFFu : lo & 0xFFu;
+        const uint32_t zp = (hi >> (8 * r)) & 0xFFu, zm = (hi >> (16 + 8 * r)) & 0xFFu;
         VX_UNROLL
         for (int x = 0; x < 8; ++x) {
             const int c = FLAT_CODE + (int((xp >> x) & 1u) - int((xm >> x) & 1u)) +
@@ -197,7 +208,6 @@ VX_HD bool block_codes(const uint32_t* occ, int block, uint8_t* code) {
             code[r * 8 + x] = uint8_t(((row >> x) & 1u) ? c : FLAT_CODE);
         }
     }
-    return any;
 }
 
 // encodeBlockTyped (DXT1Compressor.cpp:242-333) over all 16 texels (the rebuild
@@ -308,9 +318,12 @@ VX_HD void encode_coded(const uint8_t* code, CodeTable tab, uint64_t& out_a, uin
 // One block of a brick's normal payload (SVORebuild.cpp:658-722): empty texels
 // are (0,1,0); a block without occupied texels is {0, 0}.
 VX_HD void brick_block(const uint32_t* occ, int block, CodeTable tab, uint64_t& a, uint64_t& b) {
+    const uint64_t key = block_key(occ, block);
+    a = b = 0;
+    if (!key) return;
     uint8_t code[16];
-    if (block_codes(occ, block, code)) encode_coded(code, tab, a, b);
-    else a = b = 0;
+    key_codes(key, code);
+    encode_coded(code, tab, a, b);
 }
 
 }  // namespace dxtn
