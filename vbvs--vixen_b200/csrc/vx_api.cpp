@@ -145,8 +145,9 @@ int scene_alloc(const vx_octree_config& c, uint32_t node_count, uint32_t brick_c
     ds.brick_user_scale = c.max_levels - c.brick_depth;
     ds.bpa = c.bricks_per_axis;
     ds.ordinary = node_count > 0;
+    for (int i = 0; i < 3; ++i) ds.wslots[i] = ds.wsize[i] * 0.125f;
     for (int i = 0; i < 3; ++i)
-        if (!(ds.wsize[i] >= 4.0f && ds.wsize[i] <= 16384.0f && std::fabs(ds.wmin[i]) <= 1.0e5f)) ds.ordinary = 0;
+        if (!(ds.wsize[i] >= 4.0f && ds.wsize[i] <= 8.0f * float(c.bricks_per_axis) && std::fabs(ds.wmin[i]) <= 1.0e5f)) ds.ordinary = 0;
     ds.node_count = node_count;
     ds.brick_count = brick_count;
     ds.nodes = reinterpret_cast<const uint2*>(q.nodes);

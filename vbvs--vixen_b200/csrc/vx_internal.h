@@ -24,9 +24,10 @@ struct DevScene {
     int32_t min_scale;                 // 22 - max_levels + 1
     int32_t brick_user_scale;          // max_levels - brick_depth (SVOTraversal.cpp:305)
     int32_t bpa;                       // bricks per axis
-    // has nodes, sides in [4, 16384], |world_min| <= 1e5, and the brick of every
+    // has nodes, sides in [4, 8 * bpa], |world_min| <= 1e5, and the brick of every
     // grid slot has the slot's coordinates (vx_regular.cuh)
     int32_t ordinary;
+    float wslots[3];                   // wsize / 8
     uint32_t node_count, brick_count;
     const uint2* nodes;                // {child_ptr, valid | leaf << 8}
     const uint32_t* node_brick;

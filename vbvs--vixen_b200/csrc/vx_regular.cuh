@@ -47,7 +47,12 @@
 // incoherent rays with LOD 308 -> 222 us; 24-scene batched frame, primary pass
 // 1.24 -> 0.71 ms (942 M -> 570 M warp instructions), bounce pass 1.77 -> 1.22 ms.
 // Of this the branch-free march over bricks whose coordinates come from their
-// slot took 86 -> 55 us, 139 -> 120 us and 2.72 -> 2.46 ms per frame.
+// slot took 86 -> 55 us, 139 -> 120 us and 2.72 -> 2.46 ms per frame; one place
+// for the hit record and the rare quotients out of line (the bounce pass waits
+// for instructions: its lanes are all over the loop) 2.46 -> 2.26 ms per frame.
+// Tried and slower: the second form per lane instead of per warp (55.5 -> 56.8,
+// 119 -> 122 us), out of line (119 -> 124 us), or for all rays (119 -> 145 us,
+// frame 2.26 -> 2.46 ms).
 #pragma once
 #include "vx_cast.cuh"
 
@@ -89,6 +94,12 @@ __device__ __noinline__ void cast_general(const DevScene& s, float ox, float oy,
     cast_ray<LOD, true>(s, ox, oy, oz, ddx, ddy, ddz, tMinArg, tMaxArg, node, tmax, cyc, 1, h, lod);
 }
 
+// The quotients as they stand, for numerators below TINY_NUM: out of line, the
+// march hardly ever needs it.
+__device__ __noinline__ float3 tiny_quotients(float ax, float ay, float az, float dx, float dy, float dz) {
+    return make_float3(ax / dx, ay / dy, az / dz);
+}
+
 struct RegRay {
     float lo[3], d[3], rcp[3];  // grid-local origin, direction, 1 / direction (+-1e8 where |d| < 1e-8)
     float tEntry;
@@ -111,8 +122,10 @@ __device__ __forceinline__ void regular_hit(const RegRay& r, const float vmn[3],
             tn[i] = still<REG>(r.d[i]) ? -__int_as_float(0x7f800000) : div_known(a[i], r.d[i], r.rcp[i]);
         hitT = nmax(nmax3(tn[0], tn[1], tn[2]), 0.0f);  // no zero among tn: no sign of zero to keep
     } else {
+        const float3 q = tiny_quotients(a[0], a[1], a[2], r.d[0], r.d[1], r.d[2]);
+        const float qa[3] = {q.x, q.y, q.z};
 #pragma unroll
-        for (int i = 0; i < 3; ++i) tn[i] = still<REG>(r.d[i]) ? -__int_as_float(0x7f800000) : a[i] / r.d[i];
+        for (int i = 0; i < 3; ++i) tn[i] = still<REG>(r.d[i]) ? -__int_as_float(0x7f800000) : qa[i];
         hitT = gmax(gmax(gmax(tn[0], tn[1]), tn[2]), 0.0f);
     }
     const bool ax = tn[0] >= tn[1] && tn[0] >= tn[2], ay = tn[1] >= tn[2];
@@ -149,56 +162,61 @@ __device__ __forceinline__ bool regular_brick(const DevScene& s, uint32_t brick,
     float vmn[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) vmn[i] = bmn[i] + small_float(c[i]);
-    if (((bit & 32u ? w.y : w.x) >> (bit & 31u)) & 1u) {
-        regular_hit<REG>(r, vmn, c[2] * 64u + bit, h);
-        return true;
-    }
-    float tNext[3], a[3], tf[3];
+    uint32_t voxel = c[2] * 64u + bit;
+    if (!(((bit & 32u ? w.y : w.x) >> (bit & 31u)) & 1u)) {
+        float tNext[3], a[3], tf[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        a[i] = (r.d[i] > 0.0f ? vmn[i] + 1.0f : vmn[i]) - ep[i];
-        tf[i] = ((r.rcp[i] > 0.0f ? bmn[i] + 8.0f : bmn[i]) - r.lo[i]) * r.rcp[i];
-    }
-    const float tMax = nmin3(tf[0], tf[1], tf[2]);
-    if (nmin3(fabsf(a[0]), fabsf(a[1]), fabsf(a[2])) >= TINY_NUM) {
+        for (int i = 0; i < 3; ++i) {
+            a[i] = (r.d[i] > 0.0f ? vmn[i] + 1.0f : vmn[i]) - ep[i];
+            tf[i] = ((r.rcp[i] > 0.0f ? bmn[i] + 8.0f : bmn[i]) - r.lo[i]) * r.rcp[i];
+        }
+        const float tMax = nmin3(tf[0], tf[1], tf[2]);
+        if (nmin3(fabsf(a[0]), fabsf(a[1]), fabsf(a[2])) >= TINY_NUM) {
 #pragma unroll
-        for (int i = 0; i < 3; ++i) tNext[i] = still<REG>(r.d[i]) ? FLT_MAX_ : tMin + div_known(a[i], r.d[i], r.rcp[i]);
-    } else {
+            for (int i = 0; i < 3; ++i)
+                tNext[i] = still<REG>(r.d[i]) ? FLT_MAX_ : tMin + div_known(a[i], r.d[i], r.rcp[i]);
+        } else {
+            const float3 q = tiny_quotients(a[0], a[1], a[2], r.d[0], r.d[1], r.d[2]);
+            const float qa[3] = {q.x, q.y, q.z};
 #pragma unroll
-        for (int i = 0; i < 3; ++i) tNext[i] = still<REG>(r.d[i]) ? FLT_MAX_ : tMin + a[i] / r.d[i];
+            for (int i = 0; i < 3; ++i) tNext[i] = still<REG>(r.d[i]) ? FLT_MAX_ : tMin + qa[i];
+        }
+        uint32_t p = c[0] | (c[1] << 4) | (c[2] << 8);
+        const uint32_t sx = r.d[0] > 0.0f ? 1u : ~0u, sy = r.d[1] > 0.0f ? 16u : ~15u, sz = r.d[2] > 0.0f ? 256u : ~255u;
+        // Branch-free over the axes: the smallest tNext is the one the reference's
+        // comparisons pick (ties go to z, then y), and lanes that step along
+        // different axes stay together.
+        for (;;) {
+            if (nmin3(tNext[0], tNext[1], tNext[2]) > tMax) return false;
+            const bool ax = tNext[0] < tNext[1] && tNext[0] < tNext[2];
+            const bool ay = !ax && tNext[1] < tNext[2];
+            const bool az = !ax && !ay;
+            p += ax ? sx : (ay ? sy : sz);
+            if (ax) tNext[0] += fabsf(r.rcp[0]);
+            if (ay) tNext[1] += fabsf(r.rcp[1]);
+            if (az) tNext[2] += fabsf(r.rcp[2]);
+            if (p & 0x888u) return false;
+            if (az) w = __ldg(occ + (p >> 8));
+            if (((p & 0x40u ? w.y : w.x) >> ((p & 7u) | ((p >> 1) & 0x18u))) & 1u) break;
+        }
+        vmn[0] = bmn[0] + small_float(p & 7u);
+        vmn[1] = bmn[1] + small_float((p >> 4) & 7u);
+        vmn[2] = bmn[2] + small_float(p >> 8);
+        voxel = (p & 7u) | ((p >> 1) & 0x38u) | ((p >> 2) & 0x1C0u);
     }
-    uint32_t p = c[0] | (c[1] << 4) | (c[2] << 8);
-    const uint32_t sx = r.d[0] > 0.0f ? 1u : ~0u, sy = r.d[1] > 0.0f ? 16u : ~15u, sz = r.d[2] > 0.0f ? 256u : ~255u;
-    // Branch-free over the axes: the smallest tNext is the one the reference's
-    // comparisons pick (ties go to z, then y), and lanes that step along
-    // different axes stay together.
-    for (;;) {
-        if (nmin3(tNext[0], tNext[1], tNext[2]) > tMax) return false;
-        const bool ax = tNext[0] < tNext[1] && tNext[0] < tNext[2];
-        const bool ay = !ax && tNext[1] < tNext[2];
-        const bool az = !ax && !ay;
-        p += ax ? sx : (ay ? sy : sz);
-        if (ax) tNext[0] += fabsf(r.rcp[0]);
-        if (ay) tNext[1] += fabsf(r.rcp[1]);
-        if (az) tNext[2] += fabsf(r.rcp[2]);
-        if (p & 0x888u) return false;
-        if (az) w = __ldg(occ + (p >> 8));
-        if (((p & 0x40u ? w.y : w.x) >> ((p & 7u) | ((p >> 1) & 0x18u))) & 1u) break;
-    }
-    vmn[0] = bmn[0] + small_float(p & 7u);
-    vmn[1] = bmn[1] + small_float((p >> 4) & 7u);
-    vmn[2] = bmn[2] + small_float(p >> 8);
-    regular_hit<REG>(r, vmn, (p & 7u) | ((p >> 1) & 0x38u) | ((p >> 2) & 0x1C0u), h);
+    regular_hit<REG>(r, vmn, voxel, h);
     return true;
 }
 
-// The brick slot at grid position x (a lookup of handleLeafHit): x / 8
-// truncated, at most bpa - 1.  Returns its brick; DevScene::ordinary says that
-// a slot's brick has the slot's coordinates, so they need not be loaded.
+// The brick slot at slot position x >= 0 (a lookup of handleLeafHit), truncated.
+// The clamps of the lookups that cannot bind are left out: positions are at
+// most 0.999 of a side or a side - 0.001, sides are at least 4 (0.999 w <= w -
+// 0.001) and at most 8 * bpa (so the slot is below bpa).  Returns the slot's
+// brick; DevScene::ordinary says that it has the slot's coordinates, so they
+// need not be loaded.
 __device__ __forceinline__ uint32_t regular_lookup(const DevScene& s, const float x[3], uint32_t slot[3]) {
-    const int bmax = s.bpa - 1;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) slot[i] = uint32_t(imin(int(trunc_bits(x[i] * 0.125f) & 0x7FFFFFu), bmax));
+    for (int i = 0; i < 3; ++i) slot[i] = trunc_bits(x[i]) & 0x7FFFFFu;
     return grid_lookup(s, int(slot[0]), int(slot[1]), int(slot[2]));
 }
 
@@ -299,6 +317,7 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
         return REG || (cs[i] && fabsf(t) < 1000.0f) ? t : t_max_now;
     };
     int scale = ESVO_MAX_SCALE, iter = 0;
+    const int limit = imin(budget, MAX_ITER);
     const int leaf_scale = s.min_scale + s.brick_user_scale;
     uint32_t parent = 0u, pushed = 0u, entry_brick = ENTRY_UNREAD, npop = 0u, sig_pop = 0u, sig_ck = 0u;
     float exp2 = 0.5f, hh = t_max;
@@ -367,7 +386,7 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
                         const float e = (o[i] + r.d[i] * nmax(r.tEntry, 0.0f)) - s.wmin[i];
                         b = s.wsinv[i] != 0.0f ? e * s.wsinv[i] : e / s.wsize[i];
                     }
-                    x[i] = nmin(nclamp(b, 0.001f, 0.999f) * s.wsize[i], s.wsm[i]);
+                    x[i] = nclamp(b, 0.001f, 0.999f) * s.wslots[i];  // (b * wsize) / 8: the same rounding
                 }
                 uint32_t slot[3];
                 uint32_t brick = regular_lookup(s, x, slot);
@@ -378,7 +397,7 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
                         const float te0 = nmax(r.tEntry, 0.0f);
 #pragma unroll
                         for (int i = 0; i < 3; ++i)
-                            x[i] = nclamp(((o[i] + r.d[i] * te0) - s.wmin[i]) + r.d[i] * 0.01f, 0.0f, s.wsm[i]);
+                            x[i] = nclamp(((o[i] + r.d[i] * te0) - s.wmin[i]) + r.d[i] * 0.01f, 0.0f, s.wsm[i]) * 0.125f;
                         entry_brick = regular_lookup(s, x, slot);
                     }
                     brick = entry_brick;
@@ -490,8 +509,10 @@ __device__ __forceinline__ bool cast_body(const DevScene& s, const float o[3], R
                 }
             }
         }
-        if (iter >= MAX_ITER) break;
-        if (iter >= budget) return false;
+        if (iter >= limit) {
+            if (limit < MAX_ITER) return false;
+            break;
+        }
     }
     if (iter >= MAX_ITER) h.flags = F_ITER_CAP;
     return true;
