@@ -33,6 +33,8 @@ constexpr uint32_t NUM_BOUNCE_DIRS = 4096;
 
 // Cosine-weighted hemisphere directions about +z (device copy of bounce_table()).
 __device__ float g_bounce_dirs[NUM_BOUNCE_DIRS * 3];
+// Direction bin (bin_of) of table direction j turned onto a hit face: [axis | negative << 2][j].
+__device__ unsigned char g_bounce_bins[8 * NUM_BOUNCE_DIRS];
 
 struct BatchArgs {
     const DevScene* scenes;
@@ -272,25 +274,35 @@ __device__ __forceinline__ bool secondary_origin(const vx_ray& r, const vx_hit& 
     org[2] = r.oz + (r.dz * inv) * h.t;
     axis = (h.flags >> 1) & 3;
     sgn = (h.flags & VX_HIT_NORMAL_NEG) ? -1.0f : 1.0f;
-    org[axis] = org[axis] + sgn * 0.001f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (a == axis) org[a] = org[a] + sgn * 0.001f;
     return true;
 }
 
 // Bounce ray k (0 or 1) of primary ray i from its secondary origin: table
 // direction j = mix64(seed ^ mix64(2i + k)) mod 4096, its z axis turned onto
 // the hit normal.
-__device__ __forceinline__ vx_ray bounce_ray(const float org[3], int axis, float sgn, uint64_t i, uint32_t k,
-                                             uint64_t seed) {
-    const uint32_t j = uint32_t(mix64(seed ^ mix64((i << 1) | k)) & (NUM_BOUNCE_DIRS - 1));
-    const float u = g_bounce_dirs[3 * j], v = g_bounce_dirs[3 * j + 1], w = g_bounce_dirs[3 * j + 2] * sgn;
+__host__ __device__ inline uint32_t bounce_dir_of(uint64_t i, uint32_t k, uint64_t seed) {
+    return uint32_t(mix64(seed ^ mix64((i << 1) | k)) & (NUM_BOUNCE_DIRS - 1));
+}
+// Table direction (u, v, w) about +z turned onto the normal axis.
+__host__ __device__ inline void turn_dir(float u, float v, float w, int axis, float& dx, float& dy, float& dz) {
+    if (axis == 0) { dx = w; dy = u; dz = v; }
+    else if (axis == 1) { dx = v; dy = w; dz = u; }
+    else { dx = u; dy = v; dz = w; }
+}
+__device__ __forceinline__ vx_ray bounce_ray_dir(const float org[3], int axis, float sgn, uint32_t j) {
     vx_ray b;
     b.ox = org[0];
     b.oy = org[1];
     b.oz = org[2];
-    if (axis == 0) { b.dx = w; b.dy = u; b.dz = v; }
-    else if (axis == 1) { b.dx = v; b.dy = w; b.dz = u; }
-    else { b.dx = u; b.dy = v; b.dz = w; }
+    turn_dir(g_bounce_dirs[3 * j], g_bounce_dirs[3 * j + 1], g_bounce_dirs[3 * j + 2] * sgn, axis, b.dx, b.dy, b.dz);
     return b;
+}
+__device__ __forceinline__ vx_ray bounce_ray(const float org[3], int axis, float sgn, uint64_t i, uint32_t k,
+                                             uint64_t seed) {
+    return bounce_ray_dir(org, axis, sgn, bounce_dir_of(i, k, seed));
 }
 
 __global__ void spawn_bounce_kernel(const vx_ray* __restrict__ rays, const vx_hit* __restrict__ hits, uint32_t n,
@@ -347,26 +359,32 @@ struct CompactChunk {
     uint32_t start, end, scene, pad;
 };
 
-__device__ __forceinline__ uint32_t bin_of(const vx_ray& r) {
-    const uint32_t octant = uint32_t(r.dx > 0.0f) | (uint32_t(r.dy > 0.0f) << 1) | (uint32_t(r.dz > 0.0f) << 2);
-    const float ax = fabsf(r.dx), ay = fabsf(r.dy), az = fabsf(r.dz);
+__host__ __device__ inline uint32_t bin_of(float dx, float dy, float dz) {
+    const uint32_t octant = uint32_t(dx > 0.0f) | (uint32_t(dy > 0.0f) << 1) | (uint32_t(dz > 0.0f) << 2);
+    const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
     const uint32_t major = (ax >= ay && ax >= az) ? 0u : (ay >= az ? 1u : 2u);
     const uint32_t minor = (ax < ay && ax < az) ? 0u : (ay < az ? 1u : 2u);  // never equal to major
     const uint32_t next = major == 2u ? 0u : major + 1u;
     return octant * 6u + major * 2u + (minor == next ? 0u : 1u);
 }
 
-// Secondary origin of primary ray i, or false on a miss.
+// Secondary origin of primary ray i, or false on a miss.  The ray comes in three
+// 8-byte loads, of the hit its t and flag word.
 __device__ __forceinline__ bool bounce_origin(const vx_ray* __restrict__ rays, const vx_hit* __restrict__ hits,
                                               uint64_t i, float org[3], int& axis, float& sgn) {
-    const vx_ray r = rays[i];
-    const vx_hit h = hits[i];
-    return secondary_origin(r, h, org, axis, sgn);
+    const float2* p = reinterpret_cast<const float2*>(rays + i);
+    const float2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(hits) + i);
+    vx_hit h{};
+    h.t = __uint_as_float(w.x);
+    h.flags = uint8_t(w.w >> 16);
+    return secondary_origin(vx_ray{a.x, a.y, b.x, b.y, c.x, c.y}, h, org, axis, sgn);
 }
 
-// counts[c * NB + b]: bounce rays of chunk c in bin b.
+// counts[c * NB + b]: bounce rays of chunk c in bin b.  A bounce ray's bin
+// follows from the hit's face and the ray's number alone (g_bounce_bins), so
+// only the flag word of the hits is read (63 -> 35 us for 7.6 M primary rays).
 __global__ void __launch_bounds__(256) compact_count_kernel(const CompactChunk* __restrict__ chunks,
-                                                            const vx_ray* __restrict__ rays,
                                                             const vx_hit* __restrict__ hits, uint64_t seed,
                                                             uint32_t* __restrict__ counts) {
     __shared__ uint32_t hist[NB];
@@ -374,41 +392,49 @@ __global__ void __launch_bounds__(256) compact_count_kernel(const CompactChunk* 
     __syncthreads();
     const CompactChunk ch = chunks[blockIdx.x];
     for (uint32_t i = ch.start + threadIdx.x; i < ch.end; i += blockDim.x) {
-        float org[3];
-        int axis;
-        float sgn;
-        if (bounce_origin(rays, hits, i, org, axis, sgn)) {
-            atomicAdd(&hist[bin_of(bounce_ray(org, axis, sgn, i, 0, seed))], 1u);
-            atomicAdd(&hist[bin_of(bounce_ray(org, axis, sgn, i, 1, seed))], 1u);
+        const uint32_t flags = (__ldg(&reinterpret_cast<const uint4*>(hits)[i].w) >> 16) & 0xFFu;
+        if (flags & VX_HIT_HIT) {
+            const unsigned char* bins = g_bounce_bins + ((flags >> 1) & 7u) * NUM_BOUNCE_DIRS;
+            atomicAdd(&hist[bins[bounce_dir_of(i, 0, seed)]], 1u);
+            atomicAdd(&hist[bins[bounce_dir_of(i, 1, seed)]], 1u);
         }
     }
     __syncthreads();
     if (threadIdx.x < NB) counts[blockIdx.x * NB + threadIdx.x] = hist[threadIdx.x];
 }
 
-// Block s: offs[c * NB + b] = bounce rays of scene s's bin b in its chunks
-// before chunk c (an exclusive scan over the scene's chunks, one warp per
-// bin, 32 chunks at a time); tot[s * NB + b] = the bin's total.
-__global__ void __launch_bounds__(512) compact_scan_kernel(const uint32_t* __restrict__ counts,
-                                                           const uint32_t* __restrict__ first_chunk,
+// A warp per scene and bin: offs[c * NB + b] = bounce rays of scene s's bin b in
+// its chunks before chunk c (an exclusive scan over the scene's chunks, 32 at a
+// time, the counts of 128 in flight); tot[s * NB + b] = the bin's total.
+// Measured (24 scenes, 7,435 chunks) against a block per scene: 33 -> 9.5 us.
+__global__ void __launch_bounds__(256) compact_scan_kernel(const uint32_t* __restrict__ counts,
+                                                           const uint32_t* __restrict__ first_chunk, uint32_t S,
                                                            uint32_t* __restrict__ offs, uint32_t* __restrict__ tot) {
-    const uint32_t sc = blockIdx.x, lane = threadIdx.x & 31u, nwarps = blockDim.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u, job = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (job >= S * NB) return;
+    const uint32_t sc = job / NB, b = job - sc * NB;
     const uint32_t begin = first_chunk[sc], end = first_chunk[sc + 1];
-    for (uint32_t b = threadIdx.x >> 5; b < NB; b += nwarps) {
-        uint32_t run = 0;
-        for (uint32_t c0 = begin; c0 < end; c0 += 32) {
-            const uint32_t c = c0 + lane;
-            const uint32_t v = c < end ? counts[c * NB + b] : 0u;
-            uint32_t x = v;
+    uint32_t run = 0;
+    for (uint32_t c0 = begin; c0 < end; c0 += 128) {
+        uint32_t v[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t c = c0 + k * 32 + lane;
+            v[k] = c < end ? __ldg(counts + size_t(c) * NB + b) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            const uint32_t c = c0 + k * 32 + lane;
+            uint32_t x = v[k];
             for (int d = 1; d < 32; d <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
                 if (lane >= uint32_t(d)) x += y;
             }
-            if (c < end) offs[c * NB + b] = run + (x - v);
+            if (c < end) offs[size_t(c) * NB + b] = run + (x - v[k]);
             run += __shfl_sync(0xFFFFFFFFu, x, 31);
         }
-        if (lane == 0) tot[sc * NB + b] = run;
     }
+    if (lane == 0) tot[job] = run;
 }
 
 // One block: tot (S * NB totals in (scene, bin) order) becomes the exclusive
@@ -457,10 +483,19 @@ __device__ __forceinline__ void store_invalid(vx_hit* hits, uint64_t slot) {
 
 // Writes chunk c's bounce rays at base[scene * NB + b] + offs[c * NB + b] +
 // their rank in the chunk's order (k = 0 rays in primary order, then k = 1);
-// the slots of misses get the invalid record.  256 primary rays per round:
-// lanes of one bin find each other with __match_any_sync and rank by lane,
-// warp totals go through shared memory, a running count per bin crosses the
-// rounds and the two k passes.
+// the slots of misses get the invalid record.  The block sorts the chunk's
+// rays by bin first and writes them in that order, so that consecutive threads
+// write consecutive rows (each warp through 768 bytes of shared memory, a row
+// being 24 bytes).  In the chunk's order the rays are 64 groups of 32, one per
+// k, q and warp; lanes of one bin find each other with __match_any_sync, a
+// group's counts go to shared memory, one scan per bin over the groups and one
+// over the bins place them: five barriers per chunk.  Bound: DRAM.  Measured
+// (B200, 7.6 M primary and 8.5 M bounce rays) against rounds of 256 primary rays
+// per k, four barriers each, lanes writing rows of different bins: 278 -> 197 us
+// (248 us with the same three-barrier order but unsorted writes).
+constexpr uint32_t SCATTER_Q = COMPACT_CHUNK / 256;
+constexpr uint32_t SCATTER_GROUPS = 2 * COMPACT_CHUNK / 32;
+static_assert(COMPACT_CHUNK == 1024 && NUM_BOUNCE_DIRS == 4096 && NB <= 64, "a sorted ray packs into 29 bits");
 __global__ void __launch_bounds__(256) compact_scatter_kernel(const CompactChunk* __restrict__ chunks,
                                                               const vx_ray* __restrict__ rays,
                                                               const vx_hit* __restrict__ hits, uint64_t seed,
@@ -468,47 +503,121 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const CompactChunk
                                                               const uint32_t* __restrict__ base,
                                                               vx_ray* __restrict__ out, uint32_t* __restrict__ map,
                                                               vx_hit* __restrict__ bounce_hits) {
-    __shared__ uint32_t wcnt[8][NB];  // [warp][bin]
-    __shared__ uint32_t run[NB];
+    __shared__ uint16_t count[SCATTER_GROUPS][NB + 2];   // then the group's first place in its bin; padded against conflicts
+    __shared__ float org_s[3][COMPACT_CHUNK];
+    __shared__ unsigned char face_s[COMPACT_CHUNK];      // axis | negative << 2
+    __shared__ uint32_t sorted[2 * COMPACT_CHUNK];       // bin << 23 | direction << 11 | k << 10 | primary ray
+    __shared__ uint32_t start[NB + 1], place[NB];        // bin's first sorted ray, its first row less that
+    __shared__ float2 rows[8][96];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
     const CompactChunk ch = chunks[blockIdx.x];
-    if (threadIdx.x < NB) run[threadIdx.x] = base[ch.scene * NB + threadIdx.x] + offs[blockIdx.x * NB + threadIdx.x];
-    for (uint32_t k = 0; k < 2; ++k) {
-        for (uint32_t r0 = ch.start; r0 < ch.end; r0 += 256) {
-            for (uint32_t j = threadIdx.x; j < 8 * NB; j += blockDim.x) (&wcnt[0][0])[j] = 0u;
-            __syncthreads();
-            const uint32_t i = r0 + threadIdx.x;
+    for (uint32_t j = threadIdx.x; j < SCATTER_GROUPS * (NB + 2) / 2; j += 256)
+        reinterpret_cast<uint32_t*>(&count[0][0])[j] = 0u;
+    uint32_t entry[SCATTER_Q][2];  // as `sorted`; 0xFFFFFFFF: none
+#pragma unroll
+    for (uint32_t q = 0; q < SCATTER_Q; ++q) {
+        const uint32_t l = q * 256 + threadIdx.x, i = ch.start + l;
+        entry[q][0] = entry[q][1] = 0xFFFFFFFFu;
+        if (i < ch.end) {
             float org[3];
-            int axis;
-            float sgn;
-            const bool hit = i < ch.end && bounce_origin(rays, hits, i, org, axis, sgn);
-            vx_ray b{};
-            uint32_t bin = NB;  // none
-            if (hit) {
-                b = bounce_ray(org, axis, sgn, i, k, seed);
-                bin = bin_of(b);
-            }
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, bin);
-            if (hit && (peers & below) == 0) wcnt[warp][bin] = __popc(peers);  // the group's first lane
-            __syncthreads();
-            if (hit) {
-                uint32_t p = run[bin] + __popc(peers & below);
-                for (uint32_t w = 0; w < warp; ++w) p += wcnt[w][bin];
-                out[p] = b;
-                map[p] = 2 * i + k;
-            } else if (k == 0 && i < ch.end) {
+            int axis = 0;
+            float sgn = 1.0f;
+            if (bounce_origin(rays, hits, i, org, axis, sgn)) {
+                const uint32_t face = uint32_t(axis) | (sgn < 0.0f ? 4u : 0u);
+                org_s[0][l] = org[0];
+                org_s[1][l] = org[1];
+                org_s[2][l] = org[2];
+                face_s[l] = uint8_t(face);
+#pragma unroll
+                for (uint32_t k = 0; k < 2; ++k) {
+                    const uint32_t j = bounce_dir_of(i, k, seed);
+                    entry[q][k] = uint32_t(g_bounce_bins[face * NUM_BOUNCE_DIRS + j]) << 23 | j << 11 | k << 10 | l;
+                }
+            } else {
                 store_invalid(bounce_hits, 2 * uint64_t(i));
                 store_invalid(bounce_hits, 2 * uint64_t(i) + 1);
             }
-            __syncthreads();
-            if (threadIdx.x < NB) {
-                uint32_t add = 0;
-                for (uint32_t w = 0; w < 8; ++w) add += wcnt[w][threadIdx.x];
-                run[threadIdx.x] += add;
-            }
-            __syncthreads();  // the next round clears wcnt
         }
+    }
+    __syncthreads();
+    uint32_t rank[SCATTER_Q] = {};  // in the group, per k 16 bits
+#pragma unroll
+    for (uint32_t q = 0; q < SCATTER_Q; ++q)
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t bin = entry[q][k] >> 23;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, bin);
+            const uint32_t n = __popc(peers & below);
+            if (bin < NB && n == 0u) count[k * (SCATTER_GROUPS / 2) + q * 8 + warp][bin] = uint16_t(__popc(peers));
+            rank[q] |= n << (16 * k);
+        }
+    __syncthreads();
+    // exclusive scan of each bin over the groups, a warp per bin, two groups a lane; start[bin] = its total
+    for (uint32_t bin = warp; bin < NB; bin += 8) {
+        const uint32_t a = count[2 * lane][bin], b = count[2 * lane + 1][bin];
+        uint32_t x = a + b;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+            if (lane >= uint32_t(d)) x += y;
+        }
+        count[2 * lane][bin] = uint16_t(x - a - b);
+        count[2 * lane + 1][bin] = uint16_t(x - b);
+        if (lane == 31) start[bin] = x;
+    }
+    __syncthreads();
+    if (warp == 0) {  // exclusive scan over the bins, two a lane
+        const uint32_t a = 2 * lane < NB ? start[2 * lane] : 0u, b = 2 * lane + 1 < NB ? start[2 * lane + 1] : 0u;
+        uint32_t x = a + b;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+            if (lane >= uint32_t(d)) x += y;
+        }
+        __syncwarp();
+        if (lane == 31) start[NB] = x;
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j) {
+            const uint32_t bin = 2 * lane + j, at = x - a - b + (j ? a : 0u);
+            if (bin < NB) {
+                start[bin] = at;
+                place[bin] = base[ch.scene * NB + bin] + offs[blockIdx.x * NB + bin] - at;
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t q = 0; q < SCATTER_Q; ++q)
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t e = entry[q][k], bin = e >> 23;
+            if (bin < NB)
+                sorted[start[bin] + count[k * (SCATTER_GROUPS / 2) + q * 8 + warp][bin] + ((rank[q] >> (16 * k)) & 0xFFFFu)] = e;
+        }
+    __syncthreads();
+    const uint32_t total = start[NB];
+    for (uint32_t t0 = warp * 32; t0 < total; t0 += 256) {
+        const uint32_t t = t0 + lane;
+        uint32_t p = 0u;
+        if (t < total) {
+            const uint32_t e = sorted[t], l = e & 1023u;
+            p = place[e >> 23] + t;
+            const float org[3] = {org_s[0][l], org_s[1][l], org_s[2][l]};
+            const uint32_t face = face_s[l];
+            const vx_ray r = bounce_ray_dir(org, int(face & 3u), face & 4u ? -1.0f : 1.0f, (e >> 11) & 4095u);
+            rows[warp][3 * lane] = make_float2(r.ox, r.oy);
+            rows[warp][3 * lane + 1] = make_float2(r.oz, r.dx);
+            rows[warp][3 * lane + 2] = make_float2(r.dy, r.dz);
+            map[p] = 2 * (ch.start + l) + ((e >> 10) & 1u);
+        }
+        __syncwarp();
+        const uint32_t words = 3 * min(32u, total - t0);
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) {
+            const uint32_t w = j * 32 + lane, from = w / 3;
+            const uint32_t row = __shfl_sync(0xFFFFFFFFu, p, from);
+            if (w < words) reinterpret_cast<float2*>(out + row)[w - 3 * from] = rows[warp][w];
+        }
+        __syncwarp();
     }
 }
 
@@ -648,7 +757,15 @@ int ensure_bounce_table() {
     std::lock_guard<std::mutex> lk(g_table_mu);
     if (g_table_ready[dev]) return VX_OK;
     const auto& t = bounce_table();
+    std::vector<unsigned char> bins(8 * NUM_BOUNCE_DIRS, 0);
+    for (uint32_t face = 0; face < 8; ++face)
+        for (uint32_t j = 0; (face & 3u) < 3 && j < NUM_BOUNCE_DIRS; ++j) {
+            float dx, dy, dz;
+            turn_dir(t[3 * j], t[3 * j + 1], t[3 * j + 2] * (face & 4u ? -1.0f : 1.0f), int(face & 3u), dx, dy, dz);
+            bins[face * NUM_BOUNCE_DIRS + j] = uint8_t(bin_of(dx, dy, dz));
+        }
     e = cudaMemcpyToSymbol(g_bounce_dirs, t.data(), t.size() * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_bounce_bins, bins.data(), bins.size());
     if (e != cudaSuccess) return fail(VX_ECUDA, std::string("bounce table upload: ") + cudaGetErrorString(e));
     g_table_ready[dev] = true;
     return VX_OK;
@@ -1214,8 +1331,8 @@ static int capture_compact(vx_batch* b, const vx_ray* primary, const uint32_t* p
                           stream);
     if (r == VX_OK) r = record_primary_done(b, st);
     if (r == VX_OK) {
-        vx::compact_count_kernel<<<nc, 256, 0, st>>>(chunk_dev, primary, primary_hits, seed, counts);
-        vx::compact_scan_kernel<<<b->S, 512, 0, st>>>(counts, first_dev, offs, tot);
+        vx::compact_count_kernel<<<nc, 256, 0, st>>>(chunk_dev, primary_hits, seed, counts);
+        vx::compact_scan_kernel<<<(b->S * vx::NB + 7) / 8, 256, 0, st>>>(counts, first_dev, b->S, offs, tot);
         vx::compact_base_kernel<<<1, 1024, 0, st>>>(tot, b->S, cbegin);
         vx::compact_scatter_kernel<<<nc, 256, 0, st>>>(chunk_dev, primary, primary_hits, seed, offs, tot, bounce, map,
                                                        bounce_hits);
