@@ -23,7 +23,7 @@ def normal_bricks(n, seed):
     return occ
 
 
-@pytest.mark.parametrize("n", [1, 31, 2369, 9472, 30011])
+@pytest.mark.parametrize("n", [1, 31, 2369, 8191, 8192, 16383, 16384, 30011])
 def test_normals_with_result_tables(vx, cuda, n):
     import torch
     occ = normal_bricks(n, n)

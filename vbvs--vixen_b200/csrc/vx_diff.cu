@@ -278,13 +278,10 @@ extern "C" int vx_diff_backward(uint32_t n, int32_t kind, const uint32_t* dxt_id
     if ((n && (!record || !image || !target || !grad)) || (kind == 1 && !dxt_idx) || (kind != 0 && kind != 1))
         return fail(VX_EINVAL, "vx_diff_backward: bad argument");
     if (n == 0) return VX_OK;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const bool pairs = reinterpret_cast<uintptr_t>(grad) % 8 == 0;
     auto* kernel = kind == 0 ? (pairs ? diff_backward_kernel<0, true> : diff_backward_kernel<0, false>)
                              : (pairs ? diff_backward_kernel<1, true> : diff_backward_kernel<1, false>);
-    const uint32_t blocks = uint32_t(std::min<uint64_t>((uint64_t(n) + DBLOCK - 1) / DBLOCK, uint64_t(sms) * 32));
+    const uint32_t blocks = uint32_t(std::min<uint64_t>((uint64_t(n) + DBLOCK - 1) / DBLOCK, 148 * 32));
     kernel<<<blocks, DBLOCK, 0, static_cast<cudaStream_t>(stream)>>>(n, dxt_idx, record, image, target, grad, loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VX_OK : fail(VX_ECUDA, std::string("vx_diff_backward: ") + cudaGetErrorString(e));

@@ -17,6 +17,8 @@
 namespace vx {
 namespace {
 
+constexpr uint32_t SMS = 148;  // of a B200; only shapes the grids
+
 // MaterialIdToColor of every material word.  The colour is a function of the
 // id below 256 and of id % 256 above, so a block puts both tables into shared
 // memory, a plane per channel (ids of neighbouring voxels then fall in different
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(256) clear_normal_table_kernel() {
 }
 
 constexpr int NRM_WARPS = 4;
+constexpr int NRM_BLOCKS = 4;  // per SM: 3 / 4 / 5 / 6 take 0.242 / 0.228 / 0.264 / 0.274 ms for 150,001 bricks
 constexpr int NRM_WAY_BITS = 8;
 constexpr uint32_t NRM_WAYS = 1u << NRM_WAY_BITS;
 
@@ -118,9 +121,9 @@ struct NormalWarp {
     uint32_t queue_at[64];    // block's place in the warp's run
 };
 
-__global__ void __launch_bounds__(NRM_WARPS * 32) build_normals_kernel(const uint32_t* __restrict__ occ,
+__global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kernel(const uint32_t* __restrict__ occ,
                                                                        uint32_t bricks, uint32_t per_warp,
-                                                                       int shared_table, uint4* __restrict__ out) {
+                                                                       uint4* __restrict__ out) {
     extern __shared__ uint4 dyn[];
     __shared__ float4 tab[dxtn::NUM_CODES];
     const uint32_t lane = threadIdx.x & 31u;
@@ -164,11 +167,9 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) build_normals_kernel(const uin
             out[first * 32 + w.queue_at[queued + lane]] = v;
             const uint32_t h = hash(k);
             keep(k, h, v);
-            if (shared_table) {
-                const unsigned long long key = (unsigned long long)(k.x) | ((unsigned long long)(k.y) << 32);
-                slot(h)[0] = make_ulonglong2(key, normal_check(key, a, b));
-                slot(h)[1] = make_ulonglong2(a, b);
-            }
+            const unsigned long long key = (unsigned long long)(k.x) | ((unsigned long long)(k.y) << 32);
+            slot(h)[0] = make_ulonglong2(key, normal_check(key, a, b));
+            slot(h)[1] = make_ulonglong2(a, b);
         }
         __syncwarp();
     };
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) build_normals_kernel(const uin
         if (!key) out[i] = make_uint4(0u, 0u, 0u, 0u);
         else if (found) out[i] = w.block[at];
         __syncwarp();
-        if (shared_table && key && !found) {
+        if (key && !found) {
             unsigned long long a, b;
             found = read_entry(slot(h), key, a, b);
             if (found) {
@@ -204,6 +205,24 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) build_normals_kernel(const uin
     if (queued) drain(queued);
 }
 
+// Few bricks: a thread per block, no tables.  The tables pay once a brick finds
+// most of its blocks there; below that the queue's serial encodings cost more than
+// they save: 3,000 / 6,000 / 9,000 / 14,000 bricks take 21 / 31 / 45 / 68 us this
+// way and 26 / 36 / 43 / 55 us with the tables (runs of two; runs of one wave 23 / 38 /
+// 48 / 58 us).
+constexpr uint32_t NRM_DIRECT = 8192;
+__global__ void __launch_bounds__(128) build_normals_direct_kernel(const uint32_t* __restrict__ occ, uint32_t blocks,
+                                                                   uint4* __restrict__ out) {
+    __shared__ float4 tab[dxtn::NUM_CODES];
+    if (threadIdx.x < dxtn::NUM_CODES) tab[threadIdx.x] = dxtn::code_entry(int(threadIdx.x));
+    __syncthreads();
+    const uint32_t i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= blocks) return;
+    uint64_t a, b;
+    dxtn::brick_block(occ + (i >> 5) * 16, int(i & 31), dxtn::CodeTable{tab}, a, b);
+    out[i] = make_uint4(uint32_t(a), uint32_t(a >> 32), uint32_t(b), uint32_t(b >> 32));
+}
+
 // One warp per brick: the brick's 512 RGB texels (6 KiB) are copied to shared
 // memory (16-byte asynchronous copies when the colours are 16-byte aligned)
 // with a 52-word stride per 16-texel block, so that the lanes' 16-byte texel
@@ -215,6 +234,7 @@ __global__ void __launch_bounds__(NRM_WARPS * 32) build_normals_kernel(const uin
 // warp, the next brick arriving during the encoding, 0.347 ms (fewer warps fit);
 // 3 / 4 / 5 / 6 blocks per SM 0.343 / 0.337 / 0.335 / 0.339 ms.
 constexpr int DXT1_WARPS = 4;
+constexpr int DXT1_BLOCKS = 4;  // per SM
 constexpr int DXT1_STRIDE = 52;
 
 // dxt1::encode16 with the texels in pairs (dxt1::dist2 of two texels in packed
@@ -309,7 +329,7 @@ __device__ __forceinline__ uint64_t encode_block_pairs(const float* p, uint32_t 
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(DXT1_WARPS * 32, 4) build_dxt1_kernel(const float* __restrict__ rgb,
+__global__ void __launch_bounds__(DXT1_WARPS * 32, DXT1_BLOCKS) build_dxt1_kernel(const float* __restrict__ rgb,
                                                                      const uint32_t* __restrict__ occ,
                                                                      uint64_t bricks, float neg_zero,
                                                                      uint64_t* __restrict__ out) {
@@ -365,25 +385,22 @@ extern "C" int vx_build_normals_dev(const uint32_t* occ_dev, uint32_t brick_coun
     if (reinterpret_cast<uintptr_t>(occ_dev) % 16 || reinterpret_cast<uintptr_t>(out_dev) % 16)
         return fail(VX_EINVAL, "vx_build_normals_dev: buffers need 16-byte alignment");
     if (brick_count == 0) return VX_OK;
-    int dev = 0, sms = 148, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t smem = NRM_WARPS * sizeof(NormalWarp);
-    cudaError_t e = cudaFuncSetAttribute(build_normals_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, build_normals_kernel, NRM_WARPS * 32, smem);
-    if (e != cudaSuccess) return cuda_err(e, "vx_build_normals_dev");
-    // one wave of warps, each with a run of bricks
-    const uint64_t warps = uint64_t(sms) * uint64_t(std::max(1, per_sm)) * NRM_WARPS;
-    const uint32_t per_warp = uint32_t((brick_count + warps - 1) / warps);
-    const uint32_t grid = uint32_t((uint64_t(brick_count) + uint64_t(per_warp) * NRM_WARPS - 1) / (uint64_t(per_warp) * NRM_WARPS));
-    // the device-wide table pays for its clearing launch from a few bricks per warp on
-    const int shared_table = per_warp >= 4;
+    static_assert(NRM_WARPS * sizeof(NormalWarp) <= 48 * 1024, "within a launch's default shared memory");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (shared_table) clear_normal_table_kernel<<<sms, 256, 0, st>>>();
-    build_normals_kernel<<<grid, NRM_WARPS * 32, smem, st>>>(occ_dev, brick_count, per_warp, shared_table,
-                                                             reinterpret_cast<uint4*>(out_dev));
-    e = cudaGetLastError();
+    uint4* out = reinterpret_cast<uint4*>(out_dev);
+    if (brick_count < NRM_DIRECT) {
+        build_normals_direct_kernel<<<brick_count / 4 + 1, 128, 0, st>>>(occ_dev, brick_count * 32, out);
+    } else {
+        // one wave of warps, each with a run of bricks; two waves of short runs while the runs would be short anyway
+        const uint64_t warps = uint64_t(SMS) * NRM_BLOCKS * NRM_WARPS;
+        const uint32_t per_warp = brick_count < 2 * NRM_DIRECT ? 2u : uint32_t((brick_count + warps - 1) / warps);
+        const uint64_t run = uint64_t(per_warp) * NRM_WARPS;
+        clear_normal_table_kernel<<<SMS, 256, 0, st>>>();
+        build_normals_kernel<<<uint32_t((brick_count + run - 1) / run), NRM_WARPS * 32, smem, st>>>(occ_dev, brick_count,
+                                                                                                   per_warp, out);
+    }
+    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VX_OK : cuda_err(e, "vx_build_normals_dev");
 }
 
@@ -426,20 +443,14 @@ extern "C" int vx_build_dxt1_dev(const float* rgb_dev, const uint32_t* occ_dev, 
         reinterpret_cast<uintptr_t>(rgb_dev) % 4)
         return fail(VX_EINVAL, "vx_build_dxt1_dev: misaligned buffer");
     if (brick_count == 0) return VX_OK;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t smem = size_t(DXT1_WARPS) * 32 * DXT1_STRIDE * sizeof(float);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto* kernel = reinterpret_cast<uintptr_t>(rgb_dev) % 16 == 0 ? build_dxt1_kernel<true> : build_dxt1_kernel<false>;
-    int per_sm = 1;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, DXT1_WARPS * 32, smem);
-    if (e != cudaSuccess) return cuda_err(e, "vx_build_dxt1_dev");
+    static_assert(DXT1_WARPS * 32 * DXT1_STRIDE * sizeof(float) <= 48 * 1024, "within a launch's default shared memory");
     const uint32_t grid = uint32_t(std::min<uint64_t>((uint64_t(brick_count) + DXT1_WARPS - 1) / DXT1_WARPS,
-                                                      uint64_t(sms) * uint64_t(std::max(1, per_sm))));
+                                                      uint64_t(SMS) * DXT1_BLOCKS));
     kernel<<<grid, DXT1_WARPS * 32, smem, st>>>(rgb_dev, occ_dev, brick_count, -0.0f, out_dev);
-    e = cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VX_OK : cuda_err(e, "vx_build_dxt1_dev");
 }
 
@@ -506,7 +517,9 @@ extern "C" int vx_material_rgb_dev(const uint32_t* words, uint64_t n, float* rgb
     if (reinterpret_cast<uintptr_t>(words) % 4 || reinterpret_cast<uintptr_t>(rgb) % 4)
         return fail(VX_EINVAL, "vx_material_rgb_dev: misaligned buffer");
     if (n == 0) return VX_OK;
-    const unsigned blocks = unsigned(std::min<uint64_t>((n + 255) / 256, 148 * 64));
+    // one wave of blocks (each fills its tables first); more once a block has four tiles all the same
+    const uint64_t tiles = (n + 1023) / 1024;
+    const unsigned blocks = unsigned(std::max(std::min<uint64_t>(tiles, SMS * 8), std::min<uint64_t>(tiles / 4, SMS * 64)));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (reinterpret_cast<uintptr_t>(rgb) % 16 == 0) material_rgb_kernel<true><<<blocks, 256, 0, st>>>(words, n, rgb);
     else material_rgb_kernel<false><<<blocks, 256, 0, st>>>(words, n, rgb);
