@@ -10,7 +10,8 @@
 // rays of the task independently (independent thread scheduling lets lanes
 // that finish early take their next ray while others are still traversing);
 // the warp re-converges at the next task fetch.  The per-ray traversal is the
-// one of the plain kernel (vx_cast.cuh), so hits are identical bit for bit.
+// one of the plain kernel (vx_regular.cuh; vx_cast.cuh with counters), so hits
+// are identical bit for bit.
 // Static lanes may take an iteration budget: rays still running after it are
 // listed and cast again from the start by a second launch over the list.
 // The frame (vx_batch_capture_frame_compact) casts only the bounce rays of
@@ -1594,7 +1595,7 @@ static_assert(NOALLOC_TABLE_OFFSET + VX_NOALLOC_MAX_SCENES * sizeof(DevScene) <=
               "no-alloc scratch too small for its scene table");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[VX_NOALLOC_SCRATCH_BYTES];
 
-// The call's scene table travels as a kernel parameter (64 x 176 B, inside the
+// The call's scene table travels as a kernel parameter (64 x 192 B, inside the
 // 32 KB parameter limit of CUDA 12.1+), so staging it into the scratch is a
 // stream-ordered kernel: no host-to-device copy from pageable memory, which
 // would wait on the caller's stream.
