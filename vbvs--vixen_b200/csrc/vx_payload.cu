@@ -74,8 +74,10 @@ __global__ void __launch_bounds__(256) material_rgb_kernel(const uint32_t* __res
 // encodes them, one per lane.  The encoder (about 3,400 instructions) then runs
 // for some 5 % of the blocks, with all lanes busy.  Measured (B200, 150,001
 // bricks): every block encoded 0.693 ms (513 M warp instructions), the warps'
-// own tables alone 0.45 ms, with the device table 0.229 ms (81 M); 64 to 512 ways
-// per warp 0.237 / 0.234 / 0.229 / 0.278 ms.  Bound: the latency of the encoder's
+// own tables alone 0.45 ms, with the device table 0.229 ms (81 M), and 0.235 ms
+// with the warps' tables written and read in an order that the memory model
+// promises; 64 to 512 ways per warp, before that order, 0.237 / 0.234 / 0.229 /
+// 0.278 ms.  Bound: the latency of the encoder's
 // serial chain and of the table.
 //
 // The device table is one per device and nothing orders its readers and
@@ -143,22 +145,25 @@ __global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kern
     const uint32_t mult = ((blockIdx.x * NRM_WARPS + (threadIdx.x >> 5)) * 0x9E3779B2u) | 1u;
     auto way = [&](uint32_t h) { return (h * mult) >> (32 - NRM_WAY_BITS); };
     auto slot = [](uint32_t h) { return g_normal_table + 2 * size_t(h >> (32 - NRM_SLOT_BITS)); };
-    // keeps a lane's result in the warp's table (one of the lanes that share a way)
-    auto keep = [&](uint2 k, uint32_t h, uint4 v) {
-        const uint32_t group = __match_any_sync(__activemask(), way(h));
+    // Keeps a result of each of `lanes`, the lanes that call it, in the warp's table:
+    // one of the lanes that share a way writes its key and block.  The mask comes from a
+    // vote of the whole warp (or is a queue's length), never from who happens to arrive
+    // together: two parties of one branch would each elect a writer for a way, and the
+    // key of one could end up with the block of the other.
+    auto keep = [&](uint32_t lanes, uint2 k, uint32_t h, uint4 v) {
+        const uint32_t group = __match_any_sync(lanes, way(h));
         if (uint32_t(__ffs(int(group)) - 1) == lane) {
             w.key[way(h)] = k;
             w.block[way(h)] = v;
         }
     };
     uint32_t queued = 0;  // warp-uniform
-    // encodes the queue's last n <= 32 keys, one per lane
+    // encodes the queue's last n <= 32 keys, one per lane; the queue's and the table's
+    // writes before it are ordered by the caller's __syncwarp, its own by the one at its end
     auto drain = [&](uint32_t n) {
-        __syncwarp();
         queued -= n;
-        uint2 k = make_uint2(0u, 0u);
         if (lane < n) {
-            k = w.queue_key[queued + lane];
+            const uint2 k = w.queue_key[queued + lane];
             uint8_t code[16];
             dxtn::key_codes(uint64_t(k.x) | (uint64_t(k.y) << 32), code);
             uint64_t a, b;
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kern
             const uint4 v = make_uint4(uint32_t(a), uint32_t(a >> 32), uint32_t(b), uint32_t(b >> 32));
             out[first * 32 + w.queue_at[queued + lane]] = v;
             const uint32_t h = hash(k);
-            keep(k, h, v);
+            keep(0xFFFFFFFFu >> (32u - n), k, h, v);
             const unsigned long long key = (unsigned long long)(k.x) | ((unsigned long long)(k.y) << 32);
             slot(h)[0] = make_ulonglong2(key, normal_check(key, a, b));
             slot(h)[1] = make_ulonglong2(a, b);
@@ -183,15 +188,15 @@ __global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kern
         const uint64_t i = uint64_t(brick) * 32 + lane;
         if (!key) out[i] = make_uint4(0u, 0u, 0u, 0u);
         else if (found) out[i] = w.block[at];
-        __syncwarp();
-        if (key && !found) {
-            unsigned long long a, b;
-            found = read_entry(slot(h), key, a, b);
-            if (found) {
-                const uint4 v = make_uint4(uint32_t(a), uint32_t(a >> 32), uint32_t(b), uint32_t(b >> 32));
-                out[i] = v;
-                keep(k, h, v);
-            }
+        unsigned long long a = 0, b = 0;
+        const bool known = key && !found && read_entry(slot(h), key, a, b);
+        __syncwarp();  // every lane has read the warp's table, which now changes
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, known);
+        if (known) {
+            const uint4 v = make_uint4(uint32_t(a), uint32_t(a >> 32), uint32_t(b), uint32_t(b >> 32));
+            out[i] = v;
+            keep(lanes, k, h, v);
+            found = true;
         }
         const uint32_t miss = __ballot_sync(0xFFFFFFFFu, key && !found);
         if (key && !found) {
@@ -200,6 +205,7 @@ __global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kern
             w.queue_at[q] = uint32_t(i - first * 32);
         }
         queued += __popc(miss);
+        __syncwarp();  // votes order no memory: the table and the queue are read by other lanes next
         if (queued >= 32) drain(32);
     }
     if (queued) drain(queued);
