@@ -45,3 +45,18 @@ def test_the_normal_tables_writes_are_ordered_before_the_next_reads():
     assert queue > kept
     drain = body(kernel, "auto drain")
     assert "__syncwarp()" in drain[drain.index("keep("):]
+
+
+WIDTH = {"unsigned char": 1, "uint8_t": 1, "uint16_t": 2, "uint32_t": 4, "float": 4, "float2": 8, "uint2": 8,
+         "unsigned long long": 8, "uint64_t": 8, "float4": 16, "uint4": 16}
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_shared_arrays_read_by_wider_words_say_their_alignment(name):
+    """A static shared array is aligned to its elements and no more, wherever the compiler happens to
+    place it: one that is accessed through a pointer to a wider type has to ask for the alignment."""
+    text = source(name)
+    for to, array in re.findall(r"reinterpret_cast<\s*(?:const\s+)?([\w ]+?)\s*\*>\s*\(\s*&?(\w+)", text):
+        for align, of in re.findall(r"(?<!extern )__shared__\s+(?:__align__\((\d+)\)\s+)?([\w ]+?)\s+%s\s*\[" % array, text):
+            if to in WIDTH and of in WIDTH and WIDTH[to] > WIDTH[of]:
+                assert align and int(align) >= WIDTH[to], f"{name}: {array}"

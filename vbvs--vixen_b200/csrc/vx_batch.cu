@@ -504,7 +504,9 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const CompactChunk
                                                               const uint32_t* __restrict__ base,
                                                               vx_ray* __restrict__ out, uint32_t* __restrict__ map,
                                                               vx_hit* __restrict__ bounce_hits) {
-    __shared__ uint16_t count[SCATTER_GROUPS][NB + 2];   // then the group's first place in its bin; padded against conflicts
+    // then the group's first place in its bin; padded against conflicts; cleared by words
+    __shared__ __align__(4) uint16_t count[SCATTER_GROUPS][NB + 2];
+    static_assert(sizeof(count) % 4 == 0, "cleared by whole words");
     __shared__ float org_s[3][COMPACT_CHUNK];
     __shared__ unsigned char face_s[COMPACT_CHUNK];      // axis | negative << 2
     __shared__ uint32_t sorted[2 * COMPACT_CHUNK];       // bin << 23 | direction << 11 | k << 10 | primary ray
@@ -513,7 +515,7 @@ __global__ void __launch_bounds__(256) compact_scatter_kernel(const CompactChunk
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u;
     const CompactChunk ch = chunks[blockIdx.x];
-    for (uint32_t j = threadIdx.x; j < SCATTER_GROUPS * (NB + 2) / 2; j += 256)
+    for (uint32_t j = threadIdx.x; j < sizeof(count) / 4; j += 256)
         reinterpret_cast<uint32_t*>(&count[0][0])[j] = 0u;
     uint32_t entry[SCATTER_Q][2];  // as `sorted`; 0xFFFFFFFF: none
 #pragma unroll
