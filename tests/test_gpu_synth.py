@@ -36,3 +36,33 @@ def test_device_noise_rounds_like_the_host(vx, cuda, spacing, octaves, fill):
     host = vx.synth_noise(512, spacing, octaves, fill, 5, False)
     dev = vx.synth_noise_dev(512, spacing, octaves, fill, 5, False).cpu().numpy().view(np.uint64)
     np.testing.assert_array_equal(dev, host)
+
+
+def test_device_noise_from_several_threads(vx, cuda):
+    """Calls of different sizes at once, each thread on a stream of its own: every launch has the
+    shared memory its size needs, whatever size another thread launches with."""
+    import ctypes
+    import threading
+
+    import torch
+    sizes = [(512, 1 << 15, 16), (64, 16, 1), (320, 4, 3), (128, 32, 4)]
+    want = [vx.synth_noise(R, s, o, 0.3, 7, False) for R, s, o in sizes]
+    outs = [torch.zeros(R * R * (R // 64), dtype=torch.int64, device="cuda") for R, _, _ in sizes]
+    streams = [torch.cuda.Stream() for _ in sizes]
+    torch.cuda.synchronize()
+    status = [[] for _ in sizes]
+
+    def work(k):
+        R, s, o = sizes[k]
+        for _ in range(40):
+            status[k].append(vx.lib().vx_synth_noise_dev(R, s, o, 0.3, 7, 0, ctypes.c_void_p(outs[k].data_ptr()),
+                                                         ctypes.c_void_p(streams[k].cuda_stream)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert [set(x) for x in status] == [{vx.VX_OK}] * len(sizes)
+    for o, w in zip(outs, want):
+        np.testing.assert_array_equal(o.cpu().numpy().view(np.uint64), w)

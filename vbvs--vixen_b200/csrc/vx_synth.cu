@@ -39,6 +39,12 @@ constexpr uint32_t FIRST_BASE = 0x3800, FIRST_BINS = 0x4000 - FIRST_BASE;
 constexpr uint32_t HIST_BINS = 16384;
 constexpr uint32_t CAND_BUFFER = 2048;  // candidates a block gathers before it writes them out
 constexpr uint32_t LOW_BINS = 65536;
+// Dynamic shared memory the kernels may be launched with.  The rows of the octaves
+// have 4,131 cells at most (R = 2048, 16 octaves of spacings 32768 down to 1): a
+// refining histogram of 64 KiB and 8 * 4 * 4,131 bytes of cells make 197,728.  One
+// value for every call: the attribute belongs to the kernel, not to a launch, and a
+// call on another thread must find it no smaller than it needs.
+constexpr uint32_t NOISE_SMEM = 200 * 1024;
 
 struct OctDev {
     uint32_t s, cells;
@@ -426,7 +432,7 @@ static int vx_synth_noise_dev_body(uint32_t R, uint32_t spacing, uint32_t octave
     };
     auto shape = [&](auto* kernel, size_t side, Shape& out) {
         out.smem = side + p.rows * row_bytes;
-        cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(out.smem));
+        cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(NOISE_SMEM));
         int per_sm = 1;
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, out.smem);
         out.grid = uint32_t(std::min<uint64_t>(tiles, uint64_t(sms) * uint64_t(std::max(1, per_sm))));
