@@ -188,9 +188,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_refill_kernel(BatchArgs a) 
     }
 }
 
-// Static lanes.  COUNT: work counters wanted (the general iteration, which
-// keeps them); else cast_plain.
-template <int BLOCK, int MINB, bool SMEM_STACK, bool COUNT>
+// Static lanes.  GENERAL: the iteration of vx_cast.cuh, for work counters and
+// for scenes that are not DevScene::ordinary (mostly_general); else cast_plain.
+template <int BLOCK, int MINB, bool SMEM_STACK, bool GENERAL>
 __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(BatchArgs a) {
     extern __shared__ uint32_t smem[];
     DevScene* sc = reinterpret_cast<DevScene*>(smem);
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(BatchArgs a) {
             // no budget: MAX_ITER + 1, which no cast reaches (the loop stops at MAX_ITER)
             const int budget = a.budget > 0 ? a.budget : MAX_ITER + 1;
             bool ended;
-            if constexpr (COUNT)
+            if constexpr (GENERAL)
                 ended = cast_ray_budget<false, !SMEM_STACK, true>(sc[lo], p.x, p.y, q.x, q.y, w.x, w.y, a.tmin, a.tmax,
                                                                   stkN, stkT, cyc, stride, budget, h);
             else
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) batch_kernel(BatchArgs a) {
                 continue;
             }
             store_hit(a.hits, out_slot(a, r), h);
-            if constexpr (COUNT) store_counters(a.counters, out_slot(a, r), h);
+            if constexpr (GENERAL) store_counters(a.counters, out_slot(a, r), h);
         }
     }
 }
@@ -787,6 +787,7 @@ struct vx_batch {
     int per_sm[12] = {};  // resident blocks per SM of each kernel variant (0 = unresolved)
     uint32_t S = 0;
     int maxL = 1;
+    std::vector<bool> ordinary;      // per scene: DevScene::ordinary
     vx::DevScene* scenes = nullptr;  // device copy of the scene table
     uint32_t* work = nullptr;        // task counter (device scratch)
     uint32_t* retry = nullptr;       // budgeted tunings: set-aside count at [0], ray list from [64]
@@ -834,24 +835,33 @@ int cuda_err(cudaError_t e, const char* what) {
     return fail(VX_ECUDA, std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
 }
 
+// Whether static lanes take the general form for all scenes.  The plain one
+// casts the rays of a scene that is not ordinary out of line, for 1.12 (a scene
+// moved by 2^17) and 1.08 (one taller than wide) of the general form's time, and
+// those of an ordinary scene for 0.45: it pays from about one ordinary scene in
+// eight on.
+bool mostly_general(const std::vector<bool>& ordinary) {
+    return 8 * size_t(std::count(ordinary.begin(), ordinary.end(), true)) < ordinary.size();
+}
+
 size_t batch_smem(const vx_batch* b, bool smem_stack, int block) {
     size_t bytes = size_t(b->S) * sizeof(vx::DevScene) + ((size_t(b->S) + 1 + 3) & ~size_t(3)) * 4;
     if (smem_stack) bytes += (size_t(2) * size_t(b->maxL) + vx::CYC_WORDS) * size_t(block) * 4;
     return bytes;
 }
 
-template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool GENERAL>
 constexpr void (*batch_kernel_ptr())(vx::BatchArgs) {
     if constexpr (REFILL) return vx::batch_refill_kernel<BLOCK, MINB, SMEM>;
-    else return vx::batch_kernel<BLOCK, MINB, SMEM, COUNT>;
+    else return vx::batch_kernel<BLOCK, MINB, SMEM, GENERAL>;
 }
 
 // Resolves (once per batch and variant, outside any stream capture) the
 // dynamic shared-memory attribute and the resident blocks per SM.
-template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool GENERAL>
 int prepare_variant(vx_batch* b, int slot) {
     if (b->per_sm[slot]) return VX_OK;
-    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, COUNT>();
+    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, GENERAL>();
     const size_t smem = batch_smem(b, SMEM, BLOCK);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -865,10 +875,10 @@ int prepare_variant(vx_batch* b, int slot) {
     return VX_OK;
 }
 
-template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool COUNT>
+template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool GENERAL>
 int launch_variant(vx_batch* b, int slot, const vx::BatchArgs& a, cudaStream_t st) {
-    if (int r = prepare_variant<BLOCK, MINB, SMEM, REFILL, COUNT>(b, slot)) return r;
-    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, COUNT>();
+    if (int r = prepare_variant<BLOCK, MINB, SMEM, REFILL, GENERAL>(b, slot)) return r;
+    auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, GENERAL>();
     kern<<<b->num_sms * b->per_sm[slot], BLOCK, batch_smem(b, SMEM, BLOCK), st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch: launch");
@@ -877,14 +887,14 @@ int launch_variant(vx_batch* b, int slot, const vx::BatchArgs& a, cudaStream_t s
 
 template <bool PREPARE_ONLY>
 int dispatch_batch(vx_batch* b, const vx_batch_tuning& t, const vx::BatchArgs* a, cudaStream_t st) {
-    // the refilling kernels keep counters in any case; static lanes have a counting form of their own
-    const int slot = (!t.refill && a && a->counters)
+    // the refilling kernels are general and keep counters in any case; static lanes have two forms
+    const int slot = (!t.refill && ((a && a->counters) || mostly_general(b->ordinary)))
                          ? 8 + (t.block == 128 ? 0 : 2) + (t.stack_in_shared ? 0 : 1)
                          : (t.block == 128 ? 0 : 4) + (t.stack_in_shared ? 0 : 2) + (t.refill ? 1 : 0);
-#define VX_BATCH_CASE(SLOT, BLK, MINB, SMEM, REF, CNT)                                                 \
+#define VX_BATCH_CASE(SLOT, BLK, MINB, SMEM, REF, GEN)                                                 \
     case SLOT:                                                                                          \
-        return PREPARE_ONLY ? prepare_variant<BLK, MINB, SMEM, REF, CNT>(b, SLOT)                       \
-                            : launch_variant<BLK, MINB, SMEM, REF, CNT>(b, SLOT, *a, st);
+        return PREPARE_ONLY ? prepare_variant<BLK, MINB, SMEM, REF, GEN>(b, SLOT)                       \
+                            : launch_variant<BLK, MINB, SMEM, REF, GEN>(b, SLOT, *a, st);
     switch (slot) {
         VX_BATCH_CASE(0, 128, 6, true, false, false)
         VX_BATCH_CASE(1, 128, 4, true, true, true)
@@ -956,6 +966,7 @@ static int vx_batch_create_body(const vx_scene* const* scenes, uint32_t count, v
         }
         host[i] = vx::scene_dev(scenes[i]);
         b->maxL = std::max(b->maxL, host[i].max_levels);
+        b->ordinary.push_back(host[i].ordinary != 0);
     }
     b->S = count;
     cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, b->device);
@@ -1382,6 +1393,7 @@ int make_part(const vx_batch* b, uint32_t s0, uint32_t count, vx_batch** out) {
     p->device = b->device;
     p->S = count;
     p->maxL = b->maxL;
+    p->ordinary.assign(b->ordinary.begin() + s0, b->ordinary.begin() + s0 + count);
     p->tuning = b->tuning;
     p->bounce_tuning = b->bounce_tuning;
     p->num_sms = b->num_sms;
@@ -1622,7 +1634,7 @@ __global__ void __launch_bounds__(256) noalloc_stage_kernel(const __grid_constan
 struct NoallocDevice {
     bool ready = false;
     unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch on this device
-    int blocks = 0;                    // persistent grid size
+    int blocks[2] = {0, 0};            // persistent grid size, plain and general form
 };
 std::mutex g_noalloc_mu;
 NoallocDevice g_noalloc[64];
@@ -1636,19 +1648,23 @@ int noalloc_setup(int dev, NoallocDevice*& out) {
         void* ptr = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: cudaGetSymbolAddress");
-        auto kern = batch_kernel<256, 3, true, false>;
         const size_t smem_max = size_t(VX_NOALLOC_MAX_SCENES) * sizeof(DevScene) +
                                 ((size_t(VX_NOALLOC_MAX_SCENES) + 1 + 3) & ~size_t(3)) * 4 +
                                 (size_t(2) * MAX_LEVELS_ALL + CYC_WORDS) * 256 * 4;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
-        if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: shared memory attribute");
-        int per_sm = 0, sms = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem_max);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        int sms = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: occupancy");
-        if (per_sm < 1) return fail(VX_EINVAL, "vx_cast_batch_noalloc: kernel does not fit on an SM");
+        for (int general = 0; general < 2; ++general) {
+            auto* kern = general ? batch_kernel<256, 3, true, true> : batch_kernel<256, 3, true, false>;
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
+            if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: shared memory attribute");
+            int per_sm = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem_max);
+            if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: occupancy");
+            if (per_sm < 1) return fail(VX_EINVAL, "vx_cast_batch_noalloc: kernel does not fit on an SM");
+            d.blocks[general] = per_sm * sms;
+        }
         d.scratch = static_cast<unsigned char*>(ptr);
-        d.blocks = per_sm * sms;
         d.ready = true;
     }
     out = &d;
@@ -1677,12 +1693,14 @@ static int vx_cast_batch_noalloc_body(const vx_scene* const* scenes, uint32_t co
     NoallocTable table{};
     table.count = count;
     int maxL = 1;
+    std::vector<bool> ordinary;
     for (uint32_t i = 0; i < count; ++i) {
         if (!scenes[i]) return fail(VX_EINVAL, "vx_cast_batch_noalloc: null scene");
         if (scene_device(scenes[i]) != dev)
             return fail(VX_EINVAL, "vx_cast_batch_noalloc: every scene must live on the current device");
         table.scene[i] = scene_dev(scenes[i]);
         maxL = std::max(maxL, table.scene[i].max_levels);
+        ordinary.push_back(table.scene[i].ordinary != 0);
     }
     NoallocDevice* d = nullptr;
     if (int r = noalloc_setup(dev, d)) return r;
@@ -1697,7 +1715,9 @@ static int vx_cast_batch_noalloc_body(const vx_scene* const* scenes, uint32_t co
                 tmax, hits, nullptr, reinterpret_cast<uint32_t*>(d->scratch), 32u, maxL};
     const size_t smem = size_t(count) * sizeof(DevScene) + ((size_t(count) + 1 + 3) & ~size_t(3)) * 4 +
                         (size_t(2) * size_t(maxL) + CYC_WORDS) * 256 * 4;
-    batch_kernel<256, 3, true, false><<<d->blocks, 256, smem, st>>>(a);
+    const bool general = mostly_general(ordinary);
+    auto* kern = general ? batch_kernel<256, 3, true, true> : batch_kernel<256, 3, true, false>;
+    kern<<<d->blocks[general], 256, smem, st>>>(a);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: launch");
     return VX_OK;

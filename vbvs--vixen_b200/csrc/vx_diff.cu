@@ -50,7 +50,9 @@ struct Views {
     CameraDev cam[VX_DIFF_MAX_VIEWS];
 };
 
-// One pixel of the forward pass: cast, record, shade.
+// One pixel of the forward pass: cast, record, shade.  GENERAL: the scene is
+// not DevScene::ordinary (as in vx_kernels.cu).
+template <bool GENERAL>
 __device__ __forceinline__ void forward_pixel(const DevScene& s, const CameraDev& cam, uint32_t px, uint32_t py,
                                               uint32_t w, uint32_t hgt, uint32_t i, int kind,
                                               const float* __restrict__ attr, const uint32_t* __restrict__ idx,
@@ -60,7 +62,10 @@ __device__ __forceinline__ void forward_pixel(const DevScene& s, const CameraDev
     float uv_y;
     camera_ray(cam, px, py, w, hgt, r, &uv_y);
     Hit h;
-    cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, stride, MAX_ITER + 1, h);
+    if constexpr (GENERAL)
+        cast_ray(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, stride, h);
+    else
+        cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, stride, MAX_ITER + 1, h);
     store_hit(record, i, h);
     float c[3];
     if (h.flags & F_HIT) {
@@ -98,7 +103,8 @@ __device__ __forceinline__ void forward_pixel(const DevScene& s, const CameraDev
 constexpr int FWD_WARPS = VX_DIFF_FWD_WARPS;
 constexpr int FWD_THREADS = FWD_WARPS * 32;
 
-__global__ void __launch_bounds__(FWD_THREADS, 1024 / FWD_THREADS) diff_forward_kernel(
+template <bool GENERAL>
+__global__ void __launch_bounds__(FWD_THREADS, (GENERAL ? 768 : 1024) / FWD_THREADS) diff_forward_kernel(
     const __grid_constant__ DevScene s, Views views, uint32_t nviews, uint32_t w, uint32_t hgt, int kind, const float* __restrict__ attr,
     const uint32_t* __restrict__ idx, float* __restrict__ image, vx_hit* __restrict__ record) {
     extern __shared__ uint32_t smem[];
@@ -115,8 +121,8 @@ __global__ void __launch_bounds__(FWD_THREADS, 1024 / FWD_THREADS) diff_forward_
     const uint32_t px = (tl % tw) * 32 + (piece & 3u) * 8 + (lane & 7u);
     const uint32_t py = (tl / tw) * 8 + (piece >> 2) * 4 + (lane >> 3);
     if (px >= w || py >= hgt) return;
-    forward_pixel(s, views.cam[v], px, py, w, hgt, v * per_view + py * w + px, kind, attr, idx, image, record, stkN,
-                  stkT, cyc, FWD_THREADS);
+    forward_pixel<GENERAL>(s, views.cam[v], px, py, w, hgt, v * per_view + py * w + px, kind, attr, idx, image, record,
+                           stkN, stkT, cyc, FWD_THREADS);
 }
 
 // grad[0 .. 1] += (x, y) in one reduction (8-byte aligned).
@@ -282,17 +288,17 @@ extern "C" int vx_diff_forward_views(const vx_scene* scene, const vx_camera_pc* 
     Views v{};
     for (uint32_t k = 0; k < views; ++k) v.cam[k] = camera_from_pc(pcs[k]);
     const size_t smem = (size_t(2) * size_t(s.max_levels) + CYC_WORDS) * FWD_THREADS * sizeof(uint32_t);
+    auto* kernel = s.ordinary ? diff_forward_kernel<false> : diff_forward_kernel<true>;
     // stacks of scenes deeper than 15 levels need more than 48 KiB per 256 threads
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(diff_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   int(smem));
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return fail(VX_ECUDA, std::string("vx_diff_forward: ") + cudaGetErrorString(e));
     }
     const uint64_t tasks = uint64_t(views) * ((w + 31) / 32) * ((h + 7) / 8) * 8;
     const uint64_t blocks = (tasks + FWD_WARPS - 1) / FWD_WARPS;
     if (blocks > 0x7FFFFFFFull) return fail(VX_EOVERFLOW, "vx_diff_forward: too many pixels for one launch");
-    diff_forward_kernel<<<uint32_t(blocks), FWD_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(
-        s, v, views, w, h, kind, attr, dxt_idx, image, record);
+    kernel<<<uint32_t(blocks), FWD_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(s, v, views, w, h, kind, attr,
+                                                                                      dxt_idx, image, record);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VX_OK : fail(VX_ECUDA, std::string("vx_diff_forward: ") + cudaGetErrorString(e));
 }

@@ -19,15 +19,23 @@ namespace {
 constexpr int BLOCK = VX_CAST_BLOCK;
 constexpr int RENDER_WARPS = VX_RENDER_WARPS;
 constexpr int RENDER_THREADS = RENDER_WARPS * 32;
-// Threads per SM the cast and render kernels are compiled for: 1,024 leave 64
+// Threads per SM the kernels are compiled for.  Plain form: 1,024 leave 64
 // registers a thread.  At 768 / 896 / 1,024 / 1,280 threads the 1080p cave frame
 // takes 145 / 143 / 139 / 155 us, the 4K city frame with shadow rays 1.13 / 1.08 /
-// 1.05 / 1.17 ms (more warps to issue from, until spills cost more).
+// 1.05 / 1.17 ms (more warps to issue from, until spills cost more).  General
+// form, which carries more state: 896 for the cast (72 registers; at 64 it spills:
+// 0.1249 against 0.1188 ms for the cave frame), 768 for the others.
 constexpr int CAST_THREADS = 1024;
-constexpr int CAST_MIN_BLOCKS = CAST_THREADS / BLOCK;
+constexpr int GENERAL_CAST_THREADS = 896, GENERAL_THREADS = 768;
 
-template <bool LOD, bool COUNT>
-__global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays, uint32_t n,
+// Which form a launch takes: the general one (vx_cast.cuh) when counters are
+// wanted, and for a scene that is not DevScene::ordinary, none of whose rays the
+// plain form takes itself: sent through the plain kernels they would all go out of
+// line there, on 64 registers (256^3 scene moved by 2^17, 1024 x 768 rays: cast 237
+// us, this way 194; render 217 and 177, forward pass 226 and 178, incoherent rays
+// 224 and 187).
+template <bool LOD, bool GENERAL>
+__global__ void __launch_bounds__(BLOCK, (GENERAL ? GENERAL_CAST_THREADS : CAST_THREADS) / BLOCK) cast_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays, uint32_t n,
                                                       float tmin, float tmax, vx_hit* __restrict__ hits,
                                                       void* __restrict__ color,
                                                       vx_ray_counters* __restrict__ counters, LodCone lod) {
@@ -40,11 +48,11 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __gr
     const float2* r2 = reinterpret_cast<const float2*>(rays + i);
     const float2 a = __ldg(r2), b = __ldg(r2 + 1), c = __ldg(r2 + 2);
     Hit h;
-    if constexpr (COUNT) cast_ray<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h, lod);
+    if constexpr (GENERAL) cast_ray<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h, lod);
     else cast_plain<LOD>(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, MAX_ITER + 1, h, lod);
     store_hit(hits, i, h);
     if (color) store_color(s, color, i, h);
-    if constexpr (COUNT) {
+    if (GENERAL && counters) {
         uint4 rc;
         rc.x = (h.iters & 0xFFFFu) | (h.grid_reads << 16);
         rc.y = h.dda_steps;
@@ -57,10 +65,11 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_kernel(const __gr
 // The cast of rays compacted on the device: `count` (device) rays of at most
 // n_max, the hit record of ray i going to slot map[i].  The per-ray work is
 // cast_kernel's (castRay, no colour or counters).
-__global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_mapped_kernel(const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays,
-                                                                        uint32_t n_max, const uint32_t* __restrict__ count,
-                                                                        const uint32_t* __restrict__ map, float tmin,
-                                                                        float tmax, vx_hit* __restrict__ hits) {
+template <bool GENERAL>
+__global__ void __launch_bounds__(BLOCK, (GENERAL ? GENERAL_THREADS : CAST_THREADS) / BLOCK) cast_mapped_kernel(
+    const __grid_constant__ DevScene s, const vx_ray* __restrict__ rays, uint32_t n_max,
+    const uint32_t* __restrict__ count, const uint32_t* __restrict__ map, float tmin, float tmax,
+    vx_hit* __restrict__ hits) {
     extern __shared__ uint32_t smem[];
     uint32_t* stkN = smem + threadIdx.x;
     float* stkT = reinterpret_cast<float*>(smem + s.max_levels * BLOCK) + threadIdx.x;
@@ -70,7 +79,8 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_mapped_kernel(con
     const float2* r2 = reinterpret_cast<const float2*>(rays + i);
     const float2 a = __ldg(r2), b = __ldg(r2 + 1), c = __ldg(r2 + 2);
     Hit h;
-    cast_plain(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, MAX_ITER + 1, h);
+    if constexpr (GENERAL) cast_ray(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, h);
+    else cast_plain(s, a.x, a.y, b.x, b.y, c.x, c.y, tmin, tmax, stkN, stkT, cyc, BLOCK, MAX_ITER + 1, h);
     store_hit(hits, __ldg(map + i), h);
 }
 
@@ -79,7 +89,8 @@ __global__ void __launch_bounds__(BLOCK, CAST_MIN_BLOCKS) cast_mapped_kernel(con
 // neighbours in both image directions, so their traversals diverge less than
 // along a row.  Warp task t is piece t & 7 of tile t >> 3; a block holds
 // RENDER_WARPS consecutive tasks.  Outputs are indexed by pixel (y * w + x).
-__global__ void __launch_bounds__(RENDER_THREADS, CAST_THREADS / RENDER_THREADS) render_kernel(
+template <bool GENERAL>
+__global__ void __launch_bounds__(RENDER_THREADS, (GENERAL ? GENERAL_THREADS : CAST_THREADS) / RENDER_THREADS) render_kernel(
     const __grid_constant__ DevScene s, CameraDev cam, uint32_t w, uint32_t hgt, uint32_t* __restrict__ image, vx_hit* __restrict__ hits,
     void* __restrict__ color) {
     extern __shared__ uint32_t smem[];
@@ -98,7 +109,11 @@ __global__ void __launch_bounds__(RENDER_THREADS, CAST_THREADS / RENDER_THREADS)
     float uv_y;
     camera_ray(cam, px, py, w, hgt, r, &uv_y);
     Hit h;
-    cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, RENDER_THREADS, MAX_ITER + 1, h);
+    if constexpr (GENERAL)
+        cast_ray(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, RENDER_THREADS, h);
+    else
+        cast_plain(s, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, 0.0f, FLT_MAX_, stkN, stkT, cyc, RENDER_THREADS,
+                   MAX_ITER + 1, h);
     if (hits) store_hit(hits, i, h);
     if (color) store_color(s, color, i, h);
     if (image) {
@@ -185,8 +200,9 @@ int launch_cast(const DevScene& s, const vx_ray* rays, uint32_t n, float tmin, f
     const size_t smem = stack_bytes(s, BLOCK);
     const bool cone = lod && lod->ray_dir_size > 0.0f;
     const LodCone lc = cone ? LodCone{lod->ray_orig_size, lod->ray_dir_size} : LodCone{0.0f, 0.0f};
-    auto* kernel = cone ? (counters ? cast_kernel<true, true> : cast_kernel<true, false>)
-                        : (counters ? cast_kernel<false, true> : cast_kernel<false, false>);
+    const bool general = counters || !s.ordinary;
+    auto* kernel = cone ? (general ? cast_kernel<true, true> : cast_kernel<true, false>)
+                        : (general ? cast_kernel<false, true> : cast_kernel<false, false>);
     if (cudaError_t e = allow_smem(kernel, smem)) return int(e);
     kernel<<<grid, BLOCK, smem, st>>>(s, rays, n, tmin, tmax, hits, color, counters, lc);
     return int(cudaGetLastError());
@@ -196,8 +212,9 @@ int launch_cast_mapped(const DevScene& s, const vx_ray* rays, uint32_t n_max, co
                        const uint32_t* map, float tmin, float tmax, vx_hit* hits, void* stream) {
     if (n_max == 0) return int(cudaSuccess);
     const size_t smem = stack_bytes(s, BLOCK);
-    if (cudaError_t e = allow_smem(cast_mapped_kernel, smem)) return int(e);
-    cast_mapped_kernel<<<(n_max + BLOCK - 1) / BLOCK, BLOCK, smem, static_cast<cudaStream_t>(stream)>>>(
+    auto* kernel = s.ordinary ? cast_mapped_kernel<false> : cast_mapped_kernel<true>;
+    if (cudaError_t e = allow_smem(kernel, smem)) return int(e);
+    kernel<<<(n_max + BLOCK - 1) / BLOCK, BLOCK, smem, static_cast<cudaStream_t>(stream)>>>(
         s, rays, n_max, count, map, tmin, tmax, hits);
     return int(cudaGetLastError());
 }
@@ -210,9 +227,9 @@ int launch_render(const DevScene& s, const CameraDev& cam, uint32_t w, uint32_t 
     const uint64_t grid = uint64_t((w + 31) / 32) * ((h + 7) / 8) * (8 / RENDER_WARPS);
     if (grid > 0x7FFFFFFFull) return int(cudaErrorInvalidValue);
     const size_t smem = stack_bytes(s, RENDER_THREADS);
-    if (cudaError_t e = allow_smem(render_kernel, smem)) return int(e);
-    render_kernel<<<uint32_t(grid), RENDER_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(s, cam, w, h, image, hits,
-                                                                                        color);
+    auto* kernel = s.ordinary ? render_kernel<false> : render_kernel<true>;
+    if (cudaError_t e = allow_smem(kernel, smem)) return int(e);
+    kernel<<<uint32_t(grid), RENDER_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(s, cam, w, h, image, hits, color);
     return int(cudaGetLastError());
 }
 

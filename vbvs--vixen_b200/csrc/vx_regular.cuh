@@ -85,7 +85,12 @@ __device__ __forceinline__ uint32_t trunc_bits(float x) { return __float_as_uint
 __device__ __forceinline__ float small_float(uint32_t v) { return __uint_as_float(v | 0x4B000000u) - 8388608.0f; }
 
 // Rays that are not plain, out of line: the general iteration with its stack
-// in local memory.
+// in local memory.  Scenes none of whose rays are plain do not come here (their
+// launches take the general kernels); what does is rays from farther than ORD_LO,
+// the odd extreme direction and the odd scene of a batch.  Rays that are all so
+// far away (256^3 scene seen from 2e5) take 76 us this way and 59 in the general
+// kernel; with the caller's stack instead of local memory 77 to 79 us, and the
+// plain rays 1 to 2 % more.
 template <bool LOD>
 __device__ __noinline__ void cast_general(const DevScene& s, float ox, float oy, float oz, float ddx, float ddy,
                                           float ddz, float tMinArg, float tMaxArg, Hit& h, LodCone lod) {
