@@ -850,6 +850,14 @@ size_t batch_smem(const vx_batch* b, bool smem_stack, int block) {
     return bytes;
 }
 
+// Lets a kernel be launched with as much dynamic shared memory as a block of a
+// B200 may have.  The attribute belongs to the kernel: were it each batch's own
+// size, a smaller batch prepared later would refuse the larger one's launches.
+template <class K>
+cudaError_t allow_any_smem(K kernel) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
 template <int BLOCK, int MINB, bool SMEM, bool REFILL, bool GENERAL>
 constexpr void (*batch_kernel_ptr())(vx::BatchArgs) {
     if constexpr (REFILL) return vx::batch_refill_kernel<BLOCK, MINB, SMEM>;
@@ -863,12 +871,10 @@ int prepare_variant(vx_batch* b, int slot) {
     if (b->per_sm[slot]) return VX_OK;
     auto kern = batch_kernel_ptr<BLOCK, MINB, SMEM, REFILL, GENERAL>();
     const size_t smem = batch_smem(b, SMEM, BLOCK);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch: shared memory attribute");
-    }
+    cudaError_t e = allow_any_smem(kern);
+    if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch: shared memory attribute");
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BLOCK, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BLOCK, smem);
     if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch: occupancy");
     if (per_sm < 1) return fail(VX_EINVAL, "vx_cast_batch: kernel does not fit on an SM (too many scenes?)");
     b->per_sm[slot] = per_sm;
@@ -1656,7 +1662,7 @@ int noalloc_setup(int dev, NoallocDevice*& out) {
         if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: occupancy");
         for (int general = 0; general < 2; ++general) {
             auto* kern = general ? batch_kernel<256, 3, true, true> : batch_kernel<256, 3, true, false>;
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
+            e = allow_any_smem(kern);
             if (e != cudaSuccess) return cuda_err(e, "vx_cast_batch_noalloc: shared memory attribute");
             int per_sm = 0;
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem_max);
