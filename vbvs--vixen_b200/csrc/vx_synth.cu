@@ -31,6 +31,7 @@ namespace {
 constexpr uint32_t MAX_OCT = 16;
 constexpr uint32_t THREADS = 256;
 constexpr uint32_t TILE_ROWS = 8;      // rows (consecutive y, one z) per tile; R is a multiple of 64
+constexpr uint32_t QUADS = TILE_ROWS / 4;
 // Values are in [0, 2): bit patterns below 0x40000000.  The first histogram is
 // over the top 16 bits from 2^-15 up (its bin 0 takes everything below), so
 // that it needs 8 KiB per block and five blocks fit on an SM; a refining one
@@ -53,7 +54,7 @@ struct OctDev {
     const float* lat;
 };
 struct NoiseParams {
-    uint32_t R, octaves, row_cells, rows;  // row_cells: cells of all octaves; rows: of a tile (8, or 4 when 8 do not fit)
+    uint32_t R, octaves, row_cells;  // row_cells: cells of all octaves
     float neg_zero;       // -0 (vx_pairs.cuh)
     const uint2* column;  // [octave][x]: place in a row's cells, weight along x
     OctDev oct[MAX_OCT];
@@ -97,7 +98,7 @@ __global__ void lattice_kernel(NoiseParams p, float* lat, uint64_t total, uint2*
     }
 }
 
-// The values of all voxels, tile by tile (p.rows rows of one z slice, all
+// The values of all voxels, tile by tile (TILE_ROWS rows of one z slice, all
 // columns).  use(bits, x, y, z, word) gets the bit patterns of four rows y ..
 // y + 3 at column x, called by whole warps whose lanes hold 32 consecutive x;
 // word: the 32-voxel word of the first row.  after_tile() runs with the block
@@ -107,29 +108,29 @@ template <uint32_t OCT, class Use, class After>
 __device__ __forceinline__ void for_each_value(const NoiseParams& p, float4* cells, Use use, After after_tile) {
     __shared__ uint32_t row_j[MAX_OCT][TILE_ROWS], slice_k[MAX_OCT];
     __shared__ float row_w[MAX_OCT][TILE_ROWS], slice_w[MAX_OCT];
-    const uint32_t R = p.R, C = p.row_cells, rows = p.rows, quads = rows / 4;
-    const uint32_t tiles_y = R / rows;
+    const uint32_t R = p.R, C = p.row_cells;
+    const uint32_t tiles_y = R / TILE_ROWS;
     const uint32_t width = min(R, THREADS), groups = THREADS / width;  // R < 256: several quads side by side
     const uint32_t col = threadIdx.x % width, group = threadIdx.x / width;
     // cells and weights of a tile's rows and slice, read by the step along z and y only
     auto rows_of = [&](uint32_t tile) {
-        const uint32_t z = tile / tiles_y, y0 = (tile - z * tiles_y) * rows;
-        if (threadIdx.x < p.octaves * rows) {
-            const uint32_t o = threadIdx.x / rows, y = threadIdx.x % rows;
+        const uint32_t z = tile / tiles_y, y0 = (tile - z * tiles_y) * TILE_ROWS;
+        if (threadIdx.x < p.octaves * TILE_ROWS) {
+            const uint32_t o = threadIdx.x / TILE_ROWS, y = threadIdx.x % TILE_ROWS;
             cell_of(y0 + y, p.oct[o].s, row_j[o][y], row_w[o][y]);
-        } else if (threadIdx.x - p.octaves * rows < p.octaves) {
-            const uint32_t o = threadIdx.x - p.octaves * rows;
+        } else if (threadIdx.x - p.octaves * TILE_ROWS < p.octaves) {
+            const uint32_t o = threadIdx.x - p.octaves * TILE_ROWS;
             cell_of(z, p.oct[o].s, slice_k[o], slice_w[o]);
         }
     };
     if (blockIdx.x < tiles_y * R) rows_of(blockIdx.x);
     __syncthreads();
     for (uint32_t tile = blockIdx.x; tile < tiles_y * R; tile += gridDim.x) {
-        const uint32_t z = tile / tiles_y, y0 = (tile - z * tiles_y) * rows;
+        const uint32_t z = tile / tiles_y, y0 = (tile - z * tiles_y) * TILE_ROWS;
         // Along z and y, once per lattice cell and row: a thread takes a cell for
         // four rows and reads the lattice when the row's cell changes.
-        // cells[c * quads + q] holds rows 4q .. 4q + 3 of cell c.
-        for (uint32_t e = threadIdx.x; e < quads * C; e += THREADS) {
+        // cells[c * QUADS + q] holds rows 4q .. 4q + 3 of cell c.
+        for (uint32_t e = threadIdx.x; e < QUADS * C; e += THREADS) {
             const uint32_t c = e < C ? e : e - C, q = e < C ? 0u : 1u;
             uint32_t o = 0;
             while (o + 1 < p.octaves && c >= p.oct[o + 1].first) ++o;
@@ -154,7 +155,7 @@ __device__ __forceinline__ void for_each_value(const NoiseParams& p, float4* cel
                 const float ly1 = a1 + wy * (b1 - a1);
                 lz[k] = ly0 + wz * (ly1 - ly0);
             }
-            cells[c * quads + q] = make_float4(lz[0], lz[1], lz[2], lz[3]);
+            cells[c * QUADS + q] = make_float4(lz[0], lz[1], lz[2], lz[3]);
         }
         __syncthreads();
         for (uint32_t x0 = 0; x0 < R; x0 += width) {
@@ -166,16 +167,16 @@ __device__ __forceinline__ void for_each_value(const NoiseParams& p, float4* cel
                 for (uint32_t o = 0; o < OCT; ++o)
                     if (o < p.octaves) {
                         const uint2 t = __ldg(p.column + o * R + x);
-                        at[o] = cells + t.x * quads;
+                        at[o] = cells + t.x * QUADS;
                         wx[o] = make_float2(__uint_as_float(t.y), __uint_as_float(t.y));
                     }
 #pragma unroll 2
-                for (uint32_t q = group; q < quads; q += groups) {
+                for (uint32_t q = group; q < QUADS; q += groups) {
                     float2 out[2];
 #pragma unroll
                     for (uint32_t o = 0; o < OCT; ++o)
                         if (o < p.octaves) {
-                            const float4 a = at[o][q], b = at[o][quads + q];
+                            const float4 a = at[o][q], b = at[o][QUADS + q];
                             const float2 a2[2] = {make_float2(a.x, a.y), make_float2(a.z, a.w)};
                             const float2 b2[2] = {make_float2(b.x, b.y), make_float2(b.z, b.w)};
                             const float2 amp = make_float2(p.oct[o].amp, p.oct[o].amp);
@@ -420,10 +421,8 @@ static int vx_synth_noise_dev_body(uint32_t R, uint32_t spacing, uint32_t octave
     p.column = reinterpret_cast<const uint2*>(base + o_col);
     lattice_kernel<<<uint32_t(std::min<uint64_t>((at[octaves] + 255) / 256, uint64_t(sms) * 8)), 256, 0, st>>>(
         p, lat, at[octaves], reinterpret_cast<uint2*>(base + o_col), seed);
-    // persistent blocks; a tile of 8 rows unless its cells leave no room for the 64 KiB beside them
     const size_t row_bytes = size_t(p.row_cells) * 4;
-    p.rows = HIST_BINS * 4 + TILE_ROWS * row_bytes <= 200 * 1024 ? TILE_ROWS : TILE_ROWS / 2;
-    const uint64_t tiles = uint64_t(R / p.rows) * R;
+    const uint64_t tiles = uint64_t(R / TILE_ROWS) * R;
     const NoiseKernels k = kernels_for(octaves);
     // shared memory and persistent grid of a kernel with `side` bytes beside its cells
     struct Shape {
@@ -431,7 +430,7 @@ static int vx_synth_noise_dev_body(uint32_t R, uint32_t spacing, uint32_t octave
         uint32_t grid;
     };
     auto shape = [&](auto* kernel, size_t side, Shape& out) {
-        out.smem = side + p.rows * row_bytes;
+        out.smem = side + TILE_ROWS * row_bytes;
         cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(NOISE_SMEM));
         int per_sm = 1;
         if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, out.smem);
