@@ -22,16 +22,19 @@ constexpr uint32_t SMS = 148;  // of a B200; only shapes the grids
 // MaterialIdToColor of every material word.  The colour is a function of the
 // id below 256 and of id % 256 above, so a block puts both tables into shared
 // memory, a plane per channel (ids of neighbouring voxels then fall in different
-// banks), and a thread writes float `f` of the output from word f / 3.  VEC: four
-// consecutive floats as one 16-byte store (rgb 16-byte aligned).  Bound: DRAM, 16
-// bytes a word.  Measured (B200, 76.8 M words): evaluating the palette's branches
-// per word and storing channels one by one 0.531 ms, tables and 16-byte stores
-// 0.205 ms (6.0 TB/s); 16 / 32 / 64 blocks per SM 0.221 / 0.215 / 0.205 ms.
+// banks), and a thread writes float `f` of the output from word f / 3: four
+// consecutive floats as one 16-byte store, from the output's first 16-byte
+// boundary (`head` floats in) on; the floats before it and behind the last tile go
+// one by one.  Bound: DRAM, 16 bytes a word.  Measured (B200, 76.8 M words):
+// evaluating the palette's branches per word and storing channels one by one 0.531
+// ms, tables and 16-byte stores 0.205 ms (6.0 TB/s); 16 / 32 / 64 blocks per SM
+// 0.221 / 0.215 / 0.205 ms.  15.4 M words to an output off 16 bytes: single
+// stores 128 us, from the boundary on 52 us; aligned 50 us.
 constexpr uint32_t PALETTE = 512;  // ids 0..255, then the wheel of ids 256 and up
+constexpr uint32_t RGB_TILE = 768;  // 16-byte stores of a tile (1024 words), three a thread
 
-template <bool VEC>
 __global__ void __launch_bounds__(256) material_rgb_kernel(const uint32_t* __restrict__ words, uint64_t n,
-                                                           float* __restrict__ rgb) {
+                                                           uint32_t head, float* __restrict__ rgb) {
     static_assert(PALETTE % 256 == 0, "filled by whole blocks");
     __shared__ float plane[3][PALETTE];
     for (uint32_t i = threadIdx.x; i < PALETTE; i += blockDim.x) {
@@ -42,25 +45,27 @@ __global__ void __launch_bounds__(256) material_rgb_kernel(const uint32_t* __res
     }
     __syncthreads();
     auto entry = [](uint32_t id) { return id < 256u ? id : 256u + (id & 255u); };
-    // tiles of 1024 words = 768 16-byte stores, three a thread
-    const uint64_t tiles = VEC ? n / 1024 : 0;
+    const uint64_t tiles = (3 * n - head) / (4 * RGB_TILE);  // head <= 3 n
     const float* p = &plane[0][0];
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint32_t* src = words + tile * 1024;
-        float4* dst = reinterpret_cast<float4*>(rgb) + tile * 768;
+        float4* dst = reinterpret_cast<float4*>(rgb + head) + tile * RGB_TILE;
 #pragma unroll
         for (uint32_t k = 0; k < 3; ++k) {
-            const uint32_t q = k * 256 + threadIdx.x, w = 4 * q / 3;
-            const uint32_t ch = 4 * q - 3 * w;  // 0, 1 or 2: the first float's channel; the fourth has it too, a word on
+            const uint32_t q = k * 256 + threadIdx.x, f = head + 4 * q, w = f / 3;
+            const uint32_t ch = f - 3 * w;  // 0, 1 or 2: the first float's channel; the fourth has it too, a word on
             const uint32_t a = entry(__ldg(src + w)), b = entry(__ldg(src + w + 1));
             const uint32_t c1 = ch == 2u ? 0u : ch + 1u, c2 = ch == 0u ? 2u : ch - 1u;
             dst[q] = make_float4(p[ch * PALETTE + a], p[c1 * PALETTE + (ch == 2u ? b : a)],
                                  p[c2 * PALETTE + (ch == 0u ? a : b)], p[ch * PALETTE + b]);
         }
     }
-    for (uint64_t f = 3 * 1024 * tiles + blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; f < 3 * n;
-         f += uint64_t(gridDim.x) * blockDim.x)
+    const uint64_t done = 4 * RGB_TILE * tiles;
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < 3 * n - done;
+         i += uint64_t(gridDim.x) * blockDim.x) {
+        const uint64_t f = i < head ? i : i + done;
         rgb[f] = plane[f % 3][entry(__ldg(words + f / 3))];
+    }
 }
 
 // A warp takes a run of consecutive bricks, lane k block k of each.  A block's
@@ -527,8 +532,8 @@ extern "C" int vx_material_rgb_dev(const uint32_t* words, uint64_t n, float* rgb
     const uint64_t tiles = (n + 1023) / 1024;
     const unsigned blocks = unsigned(std::max(std::min<uint64_t>(tiles, SMS * 8), std::min<uint64_t>(tiles / 4, SMS * 64)));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (reinterpret_cast<uintptr_t>(rgb) % 16 == 0) material_rgb_kernel<true><<<blocks, 256, 0, st>>>(words, n, rgb);
-    else material_rgb_kernel<false><<<blocks, 256, 0, st>>>(words, n, rgb);
+    const uint32_t head = uint32_t(16 - reinterpret_cast<uintptr_t>(rgb) % 16) % 16 / 4;  // floats: at most 3 <= 3 n
+    material_rgb_kernel<<<blocks, 256, 0, st>>>(words, n, head, rgb);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? VX_OK : cuda_err(e, "vx_material_rgb_dev");
 }
