@@ -63,8 +63,17 @@ CameraDev camera_from_pc(const vx_camera_pc& pc) {
 // A host-buffer cast of at most this many rays goes through page-locked memory
 // that the kernel reads and writes itself (52 bytes a ray at most: 256 KiB per
 // scene, allocated on first use and freed with it).  A pick of one ray costs a
-// launch and a wait instead of two copies, six streams and their events: 50 -> 29
-// us through the Python binding, 256 rays 86 -> 65, 5,000 rays 157 -> 120 us.
+// launch and a wait instead of two copies, six streams and their events: 36 -> 20
+// us through the C ABI (48 -> 22 with DXT1 colours), 1,000 rays 89 -> 51 (103 -> 53),
+// 5,000 rays 97 -> 60 us (116 -> 63).
+// Why 5,000: what limits it is the buffer, not the call.  Called again and again the
+// page-locked form stays the faster one up to some 100,000 rays (10,000 rays 96 against
+// 68 us, 20,000 120 against 90, 50,000 212 against 192, 100,000 335 either way, 200,000
+// 580 against 618).  But the scene's first such call allocates the buffer, and the
+// driver cuts buffers of up to 1 MiB out of page-locked blocks of 2 MiB that take 1 to 3
+// ms each: of this size seven scenes share a block, and the first pick of the others
+// takes 73 us; with 1 MiB (20,000 rays) every second scene's takes 1.3 ms, with 16 MiB
+// every one 6.5 ms (the copies' streams and events: 1.0 ms).
 #define VX_SMALL_CAST_RAYS 5000u
 
 struct vx_scene {

@@ -1,6 +1,6 @@
 // vx_cast.cuh - the ESVO cast of one ray in its general form: casts that want
-// work counters, the refilling batched kernel, and the rays that are not plain
-// in every other cast (vx_regular.cuh).
+// work counters, scenes that are not DevScene::ordinary, the refilling batched
+// kernel, and the rays that are not plain in every other cast (vx_regular.cuh).
 //
 // One thread per ray.  The traversal restates LaineKarrasOctree::castRayImpl
 // (SVO/src/SVOTraversal.cpp:516-691), handleLeafHit and the brick DDA

@@ -139,8 +139,8 @@ __device__ __forceinline__ void add_pair(float* at, float x, float y) {
 // reductions at L2.  Measured (B200, 16 views of 512 x 512, per-voxel colours)
 // against groups of equal keys anywhere in the warp (__match_any_sync on 64
 // bits, a shuffle per lane and channel) with a block reduction per 256 pixels:
-// 162 -> 48 us; 4.2 M pixels of a closed surface 92 -> 31 us, with DXT1 endpoints
-// 165 -> 37 us.  8 / 16 / 32 blocks per SM 50 / 48 / 48 us (10.5 us with 32 for
+// 154 -> 53 us; 4.2 M pixels of a closed surface 93 -> 33 us, with DXT1 endpoints
+// 166 -> 38 us.  8 / 16 / 32 blocks per SM 50 / 48 / 48 us (10.5 us with 32 for
 // 0.4 M pixels, 13 with 8), a block per 256 pixels 76 us.
 //
 // Records need not be an image's: shuffled pixels of a few voxels, or two voxels in

@@ -20,11 +20,14 @@ constexpr int BLOCK = VX_CAST_BLOCK;
 constexpr int RENDER_WARPS = VX_RENDER_WARPS;
 constexpr int RENDER_THREADS = RENDER_WARPS * 32;
 // Threads per SM the kernels are compiled for.  Plain form: 1,024 leave 64
-// registers a thread.  At 768 / 896 / 1,024 / 1,280 threads the 1080p cave frame
-// takes 145 / 143 / 139 / 155 us, the 4K city frame with shadow rays 1.13 / 1.08 /
-// 1.05 / 1.17 ms (more warps to issue from, until spills cost more).  General
-// form, which carries more state: 896 for the cast (72 registers; at 64 it spills:
-// 0.1249 against 0.1188 ms for the cave frame), 768 for the others.
+// registers a thread.  At 768 / 896 / 1,024 / 1,152 / 1,280 threads the 1080p cave
+// frame takes 123 / 120 / 118 / 123 / 138 us, the 4K city frame with shadow rays 1.11
+// / 1.05 / 1.02 / 1.04 / 1.16 ms, incoherent rays with LOD 217 / 214 / 215 / 231 /
+// 246 us, a 1279 x 717 render 54.2 / 53.5 / 52.4 / 55.7 / 58.7 us (more warps to issue
+// from, until spills cost more); only 512 x 512 rays in pixel rows, two waves of
+// blocks, are faster at 768 (53.9 against 55.7 us).  General form, which carries more
+// state: 896 for the cast (72 registers; at 64 it spills: 0.1249 against 0.1188 ms for
+// the cave frame), 768 for the others.
 constexpr int CAST_THREADS = 1024;
 constexpr int GENERAL_CAST_THREADS = 896, GENERAL_THREADS = 768;
 

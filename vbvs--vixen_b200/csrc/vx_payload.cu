@@ -84,6 +84,13 @@ __global__ void __launch_bounds__(256) material_rgb_kernel(const uint32_t* __res
 // promises; 64 to 512 ways per warp, before that order, 0.237 / 0.234 / 0.229 /
 // 0.278 ms.  Bound: the latency of the encoder's
 // serial chain and of the table.
+// Blocks that do not repeat pay for the tables and for the fewer warps they leave
+// room for: bricks of random voxels at 50 % fill (no two blocks equal) 0.802 -> 0.946 ms
+// for 150,001 and 58 -> 74 us for 10,000, at 25 % (40 % equal) 0.681 -> 0.700 ms.  Tried
+// against it and slower on noise than it gains there: 5, 6 or 8 blocks per SM with 64
+// to 256 ways (noise 0.243 -> 0.275 .. 0.316 ms), and leaving the tables alone for six
+// bricks of eight where few blocks were found (0.930, noise 0.256 .. 0.295 ms; with an
+// encoder of its own for them 1.06, the code no longer fits the instruction cache).
 //
 // The device table is one per device and nothing orders its readers and
 // writers, warps of this call and of calls on other streams.  So an entry

@@ -3,7 +3,8 @@
 //
 // A ray is plain when the scene's world box (DevScene::ordinary), its direction
 // and its origin (ORD_LO) have ordinary sizes, so that no value is NaN; other
-// rays take cast_general, the iteration of vx_cast.cuh.  A plain ray is regular
+// rays take cast_general, the iteration of vx_cast.cuh (and launches over scenes
+// that are not ordinary take kernels made of it).  A plain ray is regular
 // when every |1 / d| is at most REG_RCP; then the octree loop needs none of the
 // reference's special cases for rays nearly parallel to an axis: every corner
 // t value is below the 1000 limit of its corrected minimum (|px - n| < 1.6
@@ -42,10 +43,10 @@
 // Bound: instruction issue, and in launches of few warps the dependent steps of
 // the longest one (descriptor, slot, voxels; then one voxel after the other).
 // Measured against the general iteration (B200): 1024^3 cave, 1920 x 1080 primary
-// rays 239 -> 120 us; 512 x 512 rays in pixel rows through a 256^3 scene
-// 123 -> 55 us; 2048^3 city at 4K with shadow rays 1.65 -> 1.05 ms; 1,000,003
-// incoherent rays with LOD 308 -> 222 us; 24-scene batched frame, primary pass
-// 1.24 -> 0.71 ms (942 M -> 570 M warp instructions), bounce pass 1.77 -> 1.22 ms.
+// rays 239 -> 118 us; 512 x 512 rays in pixel rows through a 256^3 scene
+// 123 -> 55 us; 2048^3 city at 4K with shadow rays 1.65 -> 1.02 ms; 1,000,003
+// incoherent rays with LOD 308 -> 218 us; 24-scene batched frame, primary pass
+// 1.24 -> 0.68 ms, bounce pass 1.77 -> 1.06 ms.
 // Of this the branch-free march over bricks whose coordinates come from their
 // slot took 86 -> 55 us, 139 -> 120 us and 2.72 -> 2.46 ms per frame; one place
 // for the hit record and the rare quotients out of line (the bounce pass waits
