@@ -135,8 +135,8 @@ __device__ __forceinline__ void add_pair(float* at, float x, float y) {
 // run of the warp is longer) and are added by the run's first lane.  PAIRS: the
 // gradient is 8-byte aligned, two channels per reduction.  The loss is kept per
 // thread over all its pixels and reduced once per block.
-// Bound: DRAM (record 16, image 12 and target 12 bytes a pixel) and the
-// reductions at L2.  Measured (B200, 16 views of 512 x 512, per-voxel colours)
+// Bound: the latency of its loads (record 16, image 12 and target 12 bytes a
+// pixel; DRAM 46 % busy, three quarters of the stalls) and the reductions at L2.  Measured (B200, 16 views of 512 x 512, per-voxel colours)
 // against groups of equal keys anywhere in the warp (__match_any_sync on 64
 // bits, a shuffle per lane and channel) with a block reduction per 256 pixels:
 // 154 -> 53 us; 4.2 M pixels of a closed surface 93 -> 33 us, with DXT1 endpoints

@@ -82,8 +82,9 @@ __global__ void __launch_bounds__(256) material_rgb_kernel(const uint32_t* __res
 // own tables alone 0.45 ms, with the device table 0.229 ms (81 M), and 0.235 ms
 // with the warps' tables written and read in an order that the memory model
 // promises; 64 to 512 ways per warp, before that order, 0.237 / 0.234 / 0.229 /
-// 0.278 ms.  Bound: the latency of the encoder's
-// serial chain and of the table.
+// 0.278 ms.  Bound: latency, at 36 % issue: of
+// fetching the encoder's instructions (the largest stall), of the tables' loads and of
+// the encoder's serial chain.
 // Blocks that do not repeat pay for the tables and for the fewer warps they leave
 // room for: bricks of random voxels at 50 % fill (no two blocks equal) 0.802 -> 0.946 ms
 // for 150,001 and 58 -> 74 us for 10,000, at 25 % (40 % equal) 0.681 -> 0.700 ms.  Tried
@@ -245,8 +246,8 @@ __global__ void __launch_bounds__(128) build_normals_direct_kernel(const uint32_
 // memory (16-byte asynchronous copies when the colours are 16-byte aligned)
 // with a 52-word stride per 16-texel block, so that the lanes' 16-byte texel
 // reads (lane k = block k) fall in different banks; lane k then encodes block k
-// and the warp writes its 256 output bytes contiguously.  Bound: instruction
-// issue.  Measured (B200, 150,001 bricks of materials): scalar searches with
+// and the warp writes its 256 output bytes contiguously.  Bound: the FMA pipe, whose
+// packed operations take two cycles (68 % busy, issue 56 %).  Measured (B200, 150,001 bricks of materials): scalar searches with
 // indices 0.465 ms (445 M warp instructions), pairs 0.363 ms, empty texels
 // cleared in registers instead of shared memory 0.337 ms; a second buffer per
 // warp, the next brick arriving during the encoding, 0.347 ms (fewer warps fit);
