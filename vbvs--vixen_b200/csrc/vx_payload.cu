@@ -226,9 +226,12 @@ __global__ void __launch_bounds__(NRM_WARPS * 32, NRM_BLOCKS) build_normals_kern
 
 // Few bricks: a thread per block, no tables.  The tables pay once a brick finds
 // most of its blocks there; below that the queue's serial encodings cost more than
-// they save: 3,000 / 6,000 / 9,000 / 14,000 bricks take 21 / 31 / 45 / 68 us this
-// way and 26 / 36 / 43 / 55 us with the tables (runs of two; runs of one wave 23 / 38 /
-// 48 / 58 us).
+// they save.  This way and with the tables in runs of two: 3,000 bricks 21 and 28 us;
+// 8,192 of 512^3 / 256^3 / 192^3 / 128^3 noise 40 and 40 / 42 and 47 / 42 and 48 / 44 and
+// 44; 12,000 of them 57 and 50 / 60 and 57 / 60 and 60 / 62 and 53.  Runs of one wave
+// are longer, find more in their warp's table and keep fewer warps busy: 20,000 bricks
+// of 512^3 / 256^3 noise 72 / 95 us with them and 74 / 80 in runs of two, 45,000 bricks
+// 116 / 142 and 140 / 149.
 constexpr uint32_t NRM_DIRECT = 8192;
 __global__ void __launch_bounds__(128) build_normals_direct_kernel(const uint32_t* __restrict__ occ, uint32_t blocks,
                                                                    uint4* __restrict__ out) {
