@@ -134,3 +134,54 @@ def test_general_scenes_run_the_general_kernel(vx, cuda):
             torch.cuda.synchronize()
             best[name] = min(best.get(name, 1e9), a.elapsed_time(b))
     assert best["plain call"] < 1.1 * best["with counters"], best
+
+
+@pytest.mark.parametrize("keep", [0.001, 0.05, 0.1, 0.5])
+def test_trees_with_children_beyond_their_nodes(vx, cuda, keep):
+    """A tree cut off after some of its nodes is accepted: a ray that would enter a missing child
+    stands still up to the reference's cap.  The same hits with and without counters, alone and in a
+    batch beside the whole tree, and no more time without counters than with (the plain kernel, which
+    would run the cap out, took 4 to 7 times as long)."""
+    import torch
+    from vx_b200 import workloads as W
+    bits = vx.synth_noise(256, 16, 3, 0.3, 5, False)
+    arrays = vx.build_dense(bits, 256, 8)
+    k = max(1, int(arrays.node_count * keep))
+    cut = vx.Scene(dataclasses.replace(arrays, nodes=arrays.nodes[:2 * k].copy(), node_brick=arrays.node_brick[:k].copy()))
+    whole = vx.Scene(arrays)
+    n = 200003
+    d = torch.from_numpy(W.random_rays(n, 256, seed=8)).cuda()
+    out = [torch.zeros((n, 4), dtype=torch.int32, device="cuda") for _ in range(2)]
+    counters = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
+    best = [1e9, 1e9]
+    for _ in range(6):
+        for i, c in enumerate((None, counters)):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                cut.cast_rays_dev(d, out[i], None, c)
+            b.record()
+            torch.cuda.synchronize()
+            best[i] = min(best[i], a.elapsed_time(b))
+    assert torch.equal(out[0], out[1])
+    assert best[0] < 1.1 * best[1], best
+    whole_hits = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
+    whole.cast_rays_dev(d, whole_hits)
+    batch = vx.Batch([cut, whole])
+    begin = torch.tensor([0, n, 2 * n], dtype=torch.int32, device="cuda")
+    both = torch.zeros((2 * n, 4), dtype=torch.int32, device="cuda")
+    batch.cast(torch.cat([d, d]).contiguous(), begin, both)
+    torch.cuda.synchronize()
+    assert torch.equal(both[:n], out[1]) and torch.equal(both[n:], whole_hits)
+    batch.close()
+
+
+def test_the_device_builders_children_are_nodes(vx, cuda):
+    """Scenes built on the device are taken as ordinary without a check: every child that may be
+    entered is one of their nodes."""
+    for R, levels in ((64, 6), (192, 8), (256, 8), (64, 23)):
+        bits = vx.synth_noise_dev(R, 8, 3, 0.4, R, False)
+        nodes = vx.scene_from_dense_dev(bits, R, levels).download().nodes.reshape(-1, 2)
+        inner = ~(nodes[:, 1] >> 8) & nodes[:, 1] & 0xFF
+        count = np.array([bin(v).count("1") for v in range(256)])[inner]
+        assert np.all((count == 0) | (nodes[:, 0].astype(np.int64) + count <= nodes.shape[0]))

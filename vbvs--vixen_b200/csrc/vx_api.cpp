@@ -193,8 +193,9 @@ uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
 // Host-side checks that make every device read in bounds: grid entries and
 // node brick fields are brick indices or 0xFFFFFFFF, coordinates lie in the
-// grid.  Child pointers are not rejected: the traversal bounds-checks them
-// exactly as executePushPhase does (SVOTraversal.cpp:352-354).
+// grid.  Child pointers are not rejected: the general traversal bounds-checks
+// them exactly as executePushPhase does (SVOTraversal.cpp:352-354), and a scene
+// with one beyond its nodes is not DevScene::ordinary, so it takes that one.
 int validate(const vx_scene_desc* d) {
     const vx_octree_config& c = d->config;
     if (c.brick_depth != 3) return fail(VX_EINVAL, "vx_scene_create: brick_depth must be 3 (8^3 bricks)");
@@ -265,11 +266,11 @@ int vx_scene_create(const vx_scene_desc* d, vx_scene** out) {
         uint32_t* mismatch = reinterpret_cast<uint32_t*>(static_cast<char*>(s->pool) + s->pool_bytes - 256);
         uint32_t bad = 0;
         cudaError_t e = cudaMemset(mismatch, 0, 4);
-        if (e == cudaSuccess) e = cudaError_t(vx::launch_grid_check(s->dev, mismatch, nullptr));
+        if (e == cudaSuccess) e = cudaError_t(vx::launch_ordinary_check(s->dev, mismatch, nullptr));
         if (e == cudaSuccess) e = cudaMemcpy(&bad, mismatch, 4, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) {
             vx_scene_destroy(s);
-            return vx::cuda_fail(e, "vx_scene_create: grid check");
+            return vx::cuda_fail(e, "vx_scene_create: check of grid and nodes");
         }
         if (bad) s->dev.ordinary = 0;
     }

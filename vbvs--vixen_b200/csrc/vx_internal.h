@@ -24,8 +24,8 @@ struct DevScene {
     int32_t min_scale;                 // 22 - max_levels + 1
     int32_t brick_user_scale;          // max_levels - brick_depth (SVOTraversal.cpp:305)
     int32_t bpa;                       // bricks per axis
-    // has nodes, sides in [4, 8 * bpa], |world_min| <= 1e5, and the brick of every
-    // grid slot has the slot's coordinates (vx_regular.cuh)
+    // has nodes, sides in [4, 8 * bpa], |world_min| <= 1e5, the brick of every grid
+    // slot has the slot's coordinates, and every inner child is a node (vx_regular.cuh)
     int32_t ordinary;
     float wslots[3];                   // wsize / 8
     uint32_t node_count, brick_count;
@@ -93,8 +93,8 @@ struct CameraDev {
 int launch_render(const DevScene& s, const CameraDev& cam, uint32_t w, uint32_t h, uint32_t* image,
                   vx_hit* hits, void* color, void* stream);
 // *mismatch (device, set to 0 before) becomes 1 when the brick of some grid
-// slot does not have the slot's coordinates
-int launch_grid_check(const DevScene& s, uint32_t* mismatch, void* stream);
+// slot does not have the slot's coordinates or an inner child lies beyond the nodes
+int launch_ordinary_check(const DevScene& s, uint32_t* mismatch, void* stream);
 int launch_camera_rays(const CameraDev& cam, uint32_t w, uint32_t h, vx_ray* rays, void* stream);
 // cast of device-compacted rays: min(n_max, *count) rays, ray i's record to slot map[i]
 int launch_cast_mapped(const DevScene& s, const vx_ray* rays, uint32_t n_max, const uint32_t* count,

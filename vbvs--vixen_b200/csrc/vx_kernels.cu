@@ -165,11 +165,17 @@ __global__ void __launch_bounds__(RENDER_THREADS, (GENERAL ? GENERAL_THREADS : C
     }
 }
 
-__global__ void __launch_bounds__(256) grid_check_kernel(DevScene s, uint32_t* __restrict__ mismatch) {
+__global__ void __launch_bounds__(256) ordinary_check_kernel(DevScene s, uint32_t* __restrict__ mismatch) {
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
     const uint32_t bpa = uint32_t(s.bpa), slots = bpa * bpa * bpa;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
+    for (uint32_t i = first; i < slots; i += step) {
         const uint32_t b = __ldg(s.grid + i);
         if (b != NONE && __ldg(s.coord + b) != (i % bpa | (i / bpa % bpa) << 10 | (i / (bpa * bpa)) << 20)) *mismatch = 1u;
+    }
+    for (uint64_t i = first; i < s.node_count; i += step) {
+        const uint2 nd = __ldg(s.nodes + i);
+        const uint32_t inner = ~(nd.y >> 8) & nd.y & 0xFFu;  // children that PUSH may enter
+        if (inner && uint64_t(nd.x) + uint32_t(__popc(inner)) > s.node_count) *mismatch = 1u;
     }
 }
 
@@ -236,10 +242,11 @@ int launch_render(const DevScene& s, const CameraDev& cam, uint32_t w, uint32_t 
     return int(cudaGetLastError());
 }
 
-int launch_grid_check(const DevScene& s, uint32_t* mismatch, void* stream) {
+int launch_ordinary_check(const DevScene& s, uint32_t* mismatch, void* stream) {
     const uint64_t slots = uint64_t(s.bpa) * uint64_t(s.bpa) * uint64_t(s.bpa);
-    grid_check_kernel<<<uint32_t(std::min<uint64_t>((slots + 255) / 256, 148 * 8)), 256, 0,
-                        static_cast<cudaStream_t>(stream)>>>(s, mismatch);
+    const uint64_t items = std::max<uint64_t>(slots, s.node_count);
+    ordinary_check_kernel<<<uint32_t(std::min<uint64_t>((items + 255) / 256, 148 * 8)), 256, 0,
+                            static_cast<cudaStream_t>(stream)>>>(s, mismatch);
     return int(cudaGetLastError());
 }
 
