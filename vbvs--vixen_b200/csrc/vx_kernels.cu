@@ -21,11 +21,11 @@ constexpr int RENDER_WARPS = VX_RENDER_WARPS;
 constexpr int RENDER_THREADS = RENDER_WARPS * 32;
 // Threads per SM the kernels are compiled for.  Plain form: 1,024 leave 64
 // registers a thread.  At 768 / 896 / 1,024 / 1,152 / 1,280 threads the 1080p cave
-// frame takes 123 / 120 / 118 / 123 / 138 us, the 4K city frame with shadow rays 1.11
-// / 1.05 / 1.02 / 1.04 / 1.16 ms, incoherent rays with LOD 217 / 214 / 215 / 231 /
-// 246 us, a 1279 x 717 render 54.2 / 53.5 / 52.4 / 55.7 / 58.7 us (more warps to issue
+// frame takes 123 / 119 / 116 / 123 / 139 us, the 4K city frame with shadow rays 1.10
+// / 1.04 / 1.01 / 1.04 / 1.21 ms, incoherent rays with LOD 217 / 213 / 214 / 233 /
+// 244 us, a 1279 x 717 render 53.7 / 53.0 / 52.1 / 54.8 / 58.6 us (more warps to issue
 // from, until spills cost more); only 512 x 512 rays in pixel rows, two waves of
-// blocks, are faster at 768 (53.9 against 55.7 us).  General form, which carries more
+// blocks, are faster at 768 (53.6 against 54.8 us).  General form, which carries more
 // state: 896 for the cast (72 registers; at 64 it spills: 0.1249 against 0.1188 ms for
 // the cave frame), 768 for the others.
 constexpr int CAST_THREADS = 1024;

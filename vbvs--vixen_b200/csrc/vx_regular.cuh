@@ -48,10 +48,10 @@
 // Bound: instruction issue, and in launches of few warps the dependent steps of
 // the longest one (descriptor, slot, voxels; then one voxel after the other).
 // Measured against the general iteration (B200): 1024^3 cave, 1920 x 1080 primary
-// rays 239 -> 118 us; 512 x 512 rays in pixel rows through a 256^3 scene
-// 123 -> 55 us; 2048^3 city at 4K with shadow rays 1.65 -> 1.02 ms; 1,000,003
+// rays 239 -> 116 us; 512 x 512 rays in pixel rows through a 256^3 scene
+// 123 -> 54 us; 2048^3 city at 4K with shadow rays 1.65 -> 1.00 ms; 1,000,003
 // incoherent rays with LOD 308 -> 218 us; 24-scene batched frame, primary pass
-// 1.24 -> 0.68 ms, bounce pass 1.77 -> 1.06 ms.
+// 1.24 -> 0.68 ms, bounce pass 1.77 -> 1.04 ms.
 // Of this the branch-free march over bricks whose coordinates come from their
 // slot took 86 -> 55 us, 139 -> 120 us and 2.72 -> 2.46 ms per frame; one place
 // for the hit record and the rare quotients out of line (the bounce pass waits
